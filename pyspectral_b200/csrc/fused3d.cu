@@ -25,7 +25,13 @@ template <typename T, int N, bool ROT>
 cudaError_t attrs() {
     using X = f3::XPass<T, N, ROT>;
     const int smem = (int)X::smem_bytes();
+    const int ysm = (int)f3::YTile<T, N>::SMEM;
     cudaError_t e;
+    if ((e = cudaFuncSetAttribute(f3::k3_yinv<T, N, ROT>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, ysm)) ||
+        (e = cudaFuncSetAttribute(f3::k3_yfwd<T, N, ROT>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, ysm)))
+        return e;
     if ((e = cudaFuncSetAttribute(f3::k3_x<T, N, ROT, -1>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
         return e;
@@ -42,24 +48,25 @@ cudaError_t attrs() {
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 }
 
+template <typename T, int N>
+unsigned y_grid(int nfields) {
+    using Y = f3::YTile<T, N>;
+    const long tiles = (long)(N / 2) * nfields * Y::NB;
+    return (unsigned)((tiles + Y::KT - 1) / Y::KT);
+}
+
 template <typename T, int N, bool ROT>
 cudaError_t yinv(const void* Bs, void* Bp, int nfields, const void* tw, cudaStream_t st) {
-    using D = f3::Dims<N>;
-    constexpr int per = f3::y_threads<T>() / D::T;
-    const long units = (long)N * nfields * D::NQ;
-    const unsigned grid = (unsigned)((units + per - 1) / per);
-    f3::k3_yinv<T, N, ROT><<<grid, f3::y_threads<T>(), 0, st>>>(
+    using Y = f3::YTile<T, N>;
+    f3::k3_yinv<T, N, ROT><<<y_grid<T, N>(nfields), Y::THREADS, Y::SMEM, st>>>(
         (const Pair<T>*)Bs, (Pair<T>*)Bp, nfields, (const cplx<T>*)tw);
     return cudaGetLastError();
 }
 
 template <typename T, int N, bool ROT>
 cudaError_t yfwd(const void* Bp, void* Bs, int nfields, const void* tw, cudaStream_t st) {
-    using D = f3::Dims<N>;
-    constexpr int per = f3::y_threads<T>() / D::T;
-    const long units = (long)N * nfields * D::NQ;
-    const unsigned grid = (unsigned)((units + per - 1) / per);
-    f3::k3_yfwd<T, N, ROT><<<grid, f3::y_threads<T>(), 0, st>>>(
+    using Y = f3::YTile<T, N>;
+    f3::k3_yfwd<T, N, ROT><<<y_grid<T, N>(nfields), Y::THREADS, Y::SMEM, st>>>(
         (const Pair<T>*)Bp, (Pair<T>*)Bs, nfields, (const cplx<T>*)tw);
     return cudaGetLastError();
 }

@@ -20,8 +20,8 @@
 // kz columns sharing twiddles.  B_spec interleaves x in pairs innermost,
 // B_spec[x/2][f][ky'][q][x%2] (q = kz pair), and B_phys keeps whole z lines,
 // B_phys[x][f][y][q].  An X-pass CTA holds two adjacent kz pairs of one ky' (its lanes t, t+1
-// hold x, x+1): runs of 64 bytes of B_spec.  A Y-pass CTA holds (x, x+1) x two adjacent kz
-// pairs: runs of 64 bytes of B_spec and 32 of B_phys.
+// hold x, x+1): runs of 64 bytes of B_spec.  A Y-pass tile holds (x, x+1) x four adjacent kz
+// pairs (two in fp64): runs of 128 bytes of B_spec and 64 of B_phys.
 // Each transform is one warp's (n <= 512: n/16 threads, 16 elements per thread; several
 // transforms per warp below n = 512), and its exchanges are warp-synchronised.  The state and
 // the accumulator live as compact copies of the kept modes, [c][ky'][kz][kx'] (kx' fastest, so
@@ -136,76 +136,162 @@ __device__ __forceinline__ size_t phys_idx(int x, int f, int y, int q) {
     return (((size_t)x * nslot<ROT>() + f) * N + y) * Dims<N>::NQ + q;
 }
 
-// Unit of a Y pass: (x, f, q) with x % 2 fastest, then q, f, x / 2 — the consecutive units of
-// one CTA are x, x+1 for adjacent kz pairs.
-struct YUnit {
-    int x, f, q;
-};
-template <int N>
-__device__ __forceinline__ YUnit y_unit(long unit, int nfields) {
-    const int xl = (int)(unit & 1);
-    const long rest = unit >> 1;
-    const int q = (int)(rest % Dims<N>::NQ);
-    const long r2 = rest / Dims<N>::NQ;
-    return YUnit{2 * (int)(r2 / nfields) + xl, (int)(r2 % nfields), q};
-}
-
-// Y passes: 4 warps per CTA (8 measured no faster at 512^3)
-template <typename T>
-constexpr int y_threads() { return 128; }
 // Z pass: 4 warps (fp32) or 2 (fp64), so its static shared memory stays below 48 KB
 template <typename T>
 constexpr int z_threads() { return sizeof(T) == 4 ? 128 : 64; }
 
 // ------------------------------------------------------------------------------- Y passes
+// A Y pass moves tiles of one field: (x, x+1) x QT adjacent kz pairs x every y, 128 bytes per
+// y, one Pair transform per (x, kz pair).  A tile comes into shared memory by asynchronous
+// 16-byte copies of whole rows and leaves it the same way: a warp's access covers four rows
+// of B_spec (128 bytes each) or eight 64-byte runs of B_phys, where reading the transform's
+// own pattern from global memory touched 32 lines per access (one Pair each, rows n Pairs
+// apart), and the L1 tag stage, not HBM, set the time.  The 16-byte chunks of a row are
+// XOR-swizzled by the row, so that eight lanes holding the same chunk of eight rows fall on
+// different banks; the transforms' exchanges reuse the tile's memory (n * 16 bytes per
+// sequence, the exchange of single complex values needs n * 8.5).
+// Bound now: HBM traffic in flight (512^3 fp32 Basdevant, one B200: inverse of 3 fields 0.768 ->
+// 0.388 ms = 4.6 TB/s, forward of 5 fields 0.943 -> 0.613 ms = 4.9 TB/s; 256^3 rotational 0.138
+// -> 0.074 and 0.070 -> 0.045 ms).
+template <typename T, int N>
+struct YTile {
+    using D = Dims<N>;
+    static constexpr int QT = sizeof(T) == 4 ? 4 : 2;            // kz pairs
+    static constexpr int UN = 2 * QT;                            // transforms
+    static constexpr int PT = UN * D::T;                         // threads
+    static constexpr int KT = PT >= 128 ? 1 : 128 / PT;          // tiles per CTA
+    static constexpr int THREADS = PT * KT;
+    static constexpr int NB = (D::NQ + QT - 1) / QT;             // tiles per (x pair, field)
+    static constexpr int CPP = (int)sizeof(Pair<T>) / 16;        // chunks per Pair
+    static constexpr size_t BYTES = (size_t)N * 128;
+    static constexpr size_t SMEM = KT * BYTES;
+    // shared memory holds three CTAs of 64 KB per SM (n = 512 fp32, n >= 256 fp64), 32 KB else
+    static constexpr int MIN_BLOCKS = sizeof(T) == 4 ? (THREADS > 128 ? 3 : 5) : 2;
+    static_assert(FftPlan<N>::SMEM * sizeof(cplx<T>) <= BYTES / UN, "exchange fits the tile");
+    int x2, f, q0;
+    bool active;
+    __device__ __forceinline__ YTile(long tile, int nfields) {
+        active = tile < (long)(N / 2) * nfields * NB;
+        q0 = (int)(tile % NB) * QT;
+        const long r = tile / NB;
+        f = (int)(r % nfields);
+        x2 = (int)(r / nfields);
+    }
+    // chunk position of chunk c of a row: SPEC rows (frequency side) are read by lanes two rows
+    // apart where the transform is split, by lanes on adjacent rows otherwise
+    template <bool SPEC>
+    static __device__ __forceinline__ int swz(int row, int c) {
+        if constexpr (SPEC && split_plan<N>()) return c ^ ((row >> 1) & 7);
+        else return c ^ (row & 7);
+    }
+    template <bool SPEC>
+    static __device__ __forceinline__ Pair<T> get(const unsigned char* sm, int row, int p) {
+        Pair<T> v;
+        uint4* o = reinterpret_cast<uint4*>(&v);
+#pragma unroll
+        for (int h = 0; h < CPP; ++h)
+            o[h] = *reinterpret_cast<const uint4*>(sm + row * 128 + swz<SPEC>(row, p * CPP + h) * 16);
+        return v;
+    }
+    template <bool SPEC>
+    static __device__ __forceinline__ void put(unsigned char* sm, int row, int p, const Pair<T>& v) {
+        const uint4* o = reinterpret_cast<const uint4*>(&v);
+#pragma unroll
+        for (int h = 0; h < CPP; ++h)
+            *reinterpret_cast<uint4*>(sm + row * 128 + swz<SPEC>(row, p * CPP + h) * 16) = o[h];
+    }
+    // f(row, chunk, global address) for this thread's share of the tile's valid chunks.  A row
+    // holds its Pairs as [q][x%2] on the frequency side (B_spec), [x%2][q] on the other (B_phys).
+    template <bool ROT, bool SPEC, typename B, typename F>
+    __device__ __forceinline__ void chunks(B* base, int lt, F&& fn) const {
+        constexpr int ROWS = SPEC ? D::KK : N;
+        constexpr int LANES = PT < 8 ? PT : 8;  // threads on one row (PT is a power of two)
+        static_assert(PT % LANES == 0 && 8 % LANES == 0 && LANES > 0, "rows are walked whole");
+        if (!active) return;
+#pragma unroll
+        for (int c = lt % LANES; c < 8; c += LANES) {  // once, unless PT < 8
+            const int p = c / CPP;
+            const int q = q0 + (SPEC ? p >> 1 : p % QT), xl = SPEC ? p & 1 : p / QT;
+            if (q >= D::NQ) continue;
+            B* g = base + (SPEC ? spec_idx<N, ROT>(2 * x2 + xl, f, 0, q)
+                                : phys_idx<N, ROT>(2 * x2 + xl, f, 0, q));
+            for (int row = lt / LANES; row < ROWS; row += PT / LANES)
+                fn(row, c, reinterpret_cast<uintptr_t>(g + (size_t)row * D::NQ * (SPEC ? 2 : 1)) +
+                               (c % CPP) * 16);
+        }
+    }
+    template <bool ROT, bool SPEC>
+    __device__ __forceinline__ void load(unsigned char* sm, const Pair<T>* base, int lt) const {
+        chunks<ROT, SPEC>(base, lt, [&](int row, int c, uintptr_t g) {
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                             tc::smem_u32(sm + row * 128 + swz<SPEC>(row, c) * 16)),
+                         "l"(g)
+                         : "memory");
+        });
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+    template <bool ROT, bool SPEC>
+    __device__ __forceinline__ void store(const unsigned char* sm, Pair<T>* base, int lt) const {
+        chunks<ROT, SPEC>(base, lt, [&](int row, int c, uintptr_t g) {
+            *reinterpret_cast<uint4*>(g) =
+                *reinterpret_cast<const uint4*>(sm + row * 128 + swz<SPEC>(row, c) * 16);
+        });
+    }
+};
+
 // Inverse along y of fields f < nfields: one Pair transform per (x, f, kz pair).
 template <typename T, int N, bool ROT>
-__global__ void __launch_bounds__(y_threads<T>()) k3_yinv(const Pair<T>* __restrict__ Bs,
-                                                        Pair<T>* __restrict__ Bp, int nfields,
-                                                        const cplx<T>* __restrict__ tw) {
+__global__ void __launch_bounds__(YTile<T, N>::THREADS, YTile<T, N>::MIN_BLOCKS)
+    k3_yinv(const Pair<T>* __restrict__ Bs, Pair<T>* __restrict__ Bp, int nfields,
+            const cplx<T>* __restrict__ tw) {
     using D = Dims<N>;
+    using Y = YTile<T, N>;
     constexpr int TT = D::T;
     constexpr int RIL = last_radix<N, true>();
-    __shared__ __align__(16) cplx<T> exch[y_threads<T>() / TT][FftPlan<N>::SMEM];
-    const int seq = threadIdx.x / TT, t = threadIdx.x % TT;
-    const long units = (long)N * nfields * D::NQ;
-    const long unit = (long)blockIdx.x * (y_threads<T>() / TT) + seq;
-    const bool active = unit < units;
-    const YUnit yu = y_unit<N>(unit, nfields);
-    const int x = yu.x, f = yu.f, q = yu.q;
+    extern __shared__ __align__(128) unsigned char ysm[];
+    const int kt = threadIdx.x / Y::PT, lt = threadIdx.x % Y::PT;
+    const int u = lt / TT, t = lt % TT;  // the transform: kz pair u / 2, x parity u % 2
+    const Y tile((long)blockIdx.x * Y::KT + kt, nfields);
+    unsigned char* sm = ysm + kt * Y::BYTES;
+    tile.template load<ROT, true>(sm, Bs, lt);
+    __syncthreads();
     const int kb = spec_base<N>(t), yb = phys_base<N>(t);
     Pair<T> v[16];
     for_slots([&](auto mc) {
         constexpr int M = decltype(mc)::value;
-        auto lo = [&](int k) { return Bs[spec_idx<N, ROT>(x, f, k, q)]; };
-        auto hi = [&](int k) { return Bs[spec_idx<N, ROT>(x, f, k - N + D::KK, q)]; };
-        v[M] = active ? slot_value<N, M>(kb, lo, hi, pzero<T>()) : pzero<T>();
+        auto lo = [&](int k) { return Y::template get<true>(sm, k, u); };
+        auto hi = [&](int k) { return Y::template get<true>(sm, k - N + D::KK, u); };
+        v[M] = slot_value<N, M>(kb, lo, hi, pzero<T>());
     });
-    seq_fft<N, true, true>(v, exch[seq], t, tw);
-    if (active) {
+    __syncthreads();  // the tile is in registers: its memory takes the exchanges
+    seq_fft<N, true, true>(v, reinterpret_cast<cplx<T>*>(sm + u * (Y::BYTES / Y::UN)), t, tw);
+    __syncthreads();
 #pragma unroll
-        for (int g = 0; g < 16 / RIL; ++g)
+    for (int g = 0; g < 16 / RIL; ++g)
 #pragma unroll
-            for (int m = 0; m < RIL; ++m)
-                Bp[phys_idx<N, ROT>(x, f, in_pos<N, RIL>(yb, g, m), q)] = v[g * RIL + m];
-    }
+        for (int m = 0; m < RIL; ++m)
+            Y::template put<false>(sm, in_pos<N, RIL>(yb, g, m), (u & 1) * Y::QT + (u >> 1),
+                                   v[g * RIL + m]);
+    __syncthreads();
+    tile.template store<ROT, false>(sm, Bp, lt);
 }
 
 // Forward along y of fields f < nfields, kept ky only.
 template <typename T, int N, bool ROT>
-__global__ void __launch_bounds__(y_threads<T>()) k3_yfwd(const Pair<T>* __restrict__ Bp,
-                                                        Pair<T>* __restrict__ Bs, int nfields,
-                                                        const cplx<T>* __restrict__ tw) {
+__global__ void __launch_bounds__(YTile<T, N>::THREADS, YTile<T, N>::MIN_BLOCKS)
+    k3_yfwd(const Pair<T>* __restrict__ Bp, Pair<T>* __restrict__ Bs, int nfields,
+            const cplx<T>* __restrict__ tw) {
     using D = Dims<N>;
+    using Y = YTile<T, N>;
     constexpr int TT = D::T;
     constexpr int RF0 = first_radix<N, false>();
-    __shared__ __align__(16) cplx<T> exch[y_threads<T>() / TT][FftPlan<N>::SMEM];
-    const int seq = threadIdx.x / TT, t = threadIdx.x % TT;
-    const long units = (long)N * nfields * D::NQ;
-    const long unit = (long)blockIdx.x * (y_threads<T>() / TT) + seq;
-    const bool active = unit < units;
-    const YUnit yu = y_unit<N>(unit, nfields);
-    const int x = yu.x, f = yu.f, q = yu.q;
+    extern __shared__ __align__(128) unsigned char ysm[];
+    const int kt = threadIdx.x / Y::PT, lt = threadIdx.x % Y::PT;
+    const int u = lt / TT, t = lt % TT;
+    const Y tile((long)blockIdx.x * Y::KT + kt, nfields);
+    unsigned char* sm = ysm + kt * Y::BYTES;
+    tile.template load<ROT, false>(sm, Bp, lt);
+    __syncthreads();
     const int kb = spec_base<N>(t), yb = phys_base<N>(t);
     Pair<T> v[16];
 #pragma unroll
@@ -213,14 +299,16 @@ __global__ void __launch_bounds__(y_threads<T>()) k3_yfwd(const Pair<T>* __restr
 #pragma unroll
         for (int m = 0; m < RF0; ++m)
             v[g * RF0 + m] =
-                active ? Bp[phys_idx<N, ROT>(x, f, in_pos<N, RF0>(yb, g, m), q)] : pzero<T>();
-    seq_fft<N, false, true>(v, exch[seq], t, tw);
-    if (active) {
-        for_slots([&](auto mc) {
-            constexpr int M = decltype(mc)::value;
-            slot_store<N, M>(kb, [&](int k) { Bs[spec_idx<N, ROT>(x, f, kept_of_fft<N>(k), q)] = v[M]; });
-        });
-    }
+                Y::template get<false>(sm, in_pos<N, RF0>(yb, g, m), (u & 1) * Y::QT + (u >> 1));
+    __syncthreads();
+    seq_fft<N, false, true>(v, reinterpret_cast<cplx<T>*>(sm + u * (Y::BYTES / Y::UN)), t, tw);
+    __syncthreads();
+    for_slots([&](auto mc) {
+        constexpr int M = decltype(mc)::value;
+        slot_store<N, M>(kb, [&](int k) { Y::template put<true>(sm, kept_of_fft<N>(k), u, v[M]); });
+    });
+    __syncthreads();
+    tile.template store<ROT, true>(sm, Bs, lt);
 }
 
 // ------------------------------------------------------------------------------- Z pass

@@ -71,6 +71,34 @@ def test_fused3d_128_matches_oracle(form):
     assert rel(s.get_state(), ref.get_state()) < 1e-12
 
 
+@pytest.mark.parametrize("n,dtype", [(16, "float64"), (32, "float32"), (128, "float32"),
+                                     (256, "float32"), (256, "float64")])
+@pytest.mark.parametrize("form", ["basdevant", "rotational"])
+def test_fused3d_y_tiles_match_the_general_engine(n, dtype, form):
+    """The Y passes' tiles (x pair x adjacent kz pairs) at the edges of their shapes: fewer
+    threads than a row has chunks (16, fp64), a partial last tile (32 and 128, fp32), several
+    tiles per CTA, one tile per CTA (256, fp32).  One step from a random field with no zero
+    component against the fp64 cuFFT engine from the same state."""
+    import torch
+
+    cfg = Config(n=n, dim=3, nu=1e-2, dtype=dtype, form=form)
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    ic = torch.fft.rfftn(torch.randn((3, n, n, n), generator=gen, device="cuda",
+                                     dtype=torch.float64), dim=(1, 2, 3))
+    k = torch.fft.fftfreq(n, 1.0 / n, device="cuda", dtype=torch.float64)
+    kz = torch.arange(n // 2 + 1, device="cuda", dtype=torch.float64)
+    k2 = k[:, None, None] ** 2 + k[None, :, None] ** 2 + kz[None, None, :] ** 2
+    ic *= torch.exp(-k2 / (n / 6.0) ** 2)
+    out = {}
+    for name, c in ((FUSED, cfg), ("b200", cfg.with_(dtype="float64"))):
+        s = get(name).make(c)
+        s.set_state(ic)
+        s.step(0.2 / n)
+        out[name] = s.state_native().to(torch.complex128).clone()
+    err = float((out[FUSED] - out["b200"]).abs().max() / out["b200"].abs().max())
+    assert err < TOL[dtype], err
+
+
 @pytest.mark.parametrize("form", ["basdevant", "rotational"])
 def test_fused3d_cfl_and_diagnostics_match_the_oracle(form):
     n = 32
