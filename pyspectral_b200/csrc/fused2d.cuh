@@ -249,19 +249,21 @@ __global__ void __launch_bounds__(RowPairs<N>::THREADS) k_row_max(const Pair<T>*
             v[g * RI + m] = Pair<T>{row_input<T, N>(X, p, k, kc, 0), row_input<T, N>(X, p, k, kc, 1)};
         }
     seq_fft<N, true>(v, sm, t, tw);
-    double mu = 0.0, mv = 0.0;
+    // in the real type itself (the maximum is exact): fp64 conversions of every sample ran at a
+    // sixteenth of the fp32 rate
+    T mu = 0, mv = 0;
     bool nan_u = false, nan_v = false;
 #pragma unroll
     for (int e = 0; e < 16; ++e) {
-        const double a0 = (double)v[e].a.x, b0 = (double)v[e].a.y;
-        const double a1 = (double)v[e].b.x, b1 = (double)v[e].b.y;
+        const T a0 = v[e].a.x, b0 = v[e].a.y;
+        const T a1 = v[e].b.x, b1 = v[e].b.y;
         nan_u |= (a0 != a0) || (a1 != a1);
         nan_v |= (b0 != b0) || (b1 != b1);
         mu = fmax(mu, fmax(fabs(a0), fabs(a1)));
         mv = fmax(mv, fmax(fabs(b0), fabs(b1)));
     }
-    unsigned long long bu = (unsigned long long)__double_as_longlong(mu);
-    unsigned long long bv = (unsigned long long)__double_as_longlong(mv);
+    unsigned long long bu = (unsigned long long)__double_as_longlong((double)mu);
+    unsigned long long bv = (unsigned long long)__double_as_longlong((double)mv);
     // a NaN anywhere wins the max, as in a NaN-propagating maximum
     if (nan_u) bu = 0x7ff8000000000000ull;
     if (nan_v) bv = 0x7ff8000000000000ull;
