@@ -327,7 +327,7 @@ __device__ __forceinline__ unsigned long long max_bits(double m, bool nan) {
 // are paired (velocities, vorticities, stresses), as the transform along z pairs them.
 // The pass is bound by instruction issue: with the half spectra stored instead (two reads and
 // four adds per completed value, two exchanges through shared memory to split the outputs)
-// 512^3 fp32 Basdevant took 1.29 ms, now 1.03; 256^3 rotational 0.121 -> 0.113 ms.
+// 512^3 fp32 Basdevant took 1.29 ms, now 1.09; 256^3 rotational 0.121 -> 0.114 ms.
 template <typename C>
 __device__ __forceinline__ C conj(C z) {
     z.y = -z.y;
@@ -531,6 +531,12 @@ __global__ void __launch_bounds__(z_threads<T>()) k3_z(Pair<T>* __restrict__ Bp,
 // slot), each warp SEQ transforms.  U = 2 (two adjacent kz pairs) except in fp64 at n = 512,
 // where the shared memory holds one.  STAGE -1: the stage-0 inputs from the state (no forward
 // transform, no update).
+// Shared memory holds one row of kept kx per (unit, field); a transform exchanges through the
+// row it will write (forward) or has read (inverse), so the rows are all the memory there is
+// and registers, not shared memory, set the resident CTAs.  The update's state and accumulator
+// are loaded one element ahead.  Bound: latency (load, transform, update, transform in a row) at
+// 18-20 warps per SM.  512^3 fp32 Basdevant 1.18 -> 1.11 ms, 256^3 rotational 0.140 -> 0.124
+// ms, 128^3 fp64 rotational 0.049 -> 0.038 ms per launch.
 template <typename T, int N, bool ROT>
 struct XPass {
     using D = Dims<N>;
@@ -539,17 +545,15 @@ struct XPass {
     // SM, which leaves the pass its registers (two pairs of 12 warps at two CTAs spill)
     static constexpr bool ONE_PAIR_ROT = ROT && sizeof(T) == 4 && S == 1;
     static constexpr int G = (S >= 2 || sizeof(T) == 8 || ONE_PAIR_ROT) ? 1 : 2;
-    static constexpr int MIN_BLOCKS = ONE_PAIR_ROT ? 3 : 2;
     static constexpr int U = G * S;
     static constexpr int WARPS = G * nslot<ROT>();
     static constexpr int THREADS = WARPS * 32;
-    static constexpr size_t stage_bytes() {
-        return (size_t)U * nslot<ROT>() * D::KK * sizeof(Pair<T>);
-    }
-    static constexpr size_t smem_bytes() {
-        return stage_bytes() + (size_t)WARPS * S * FftPlan<N>::SMEM * sizeof(cplx<T>);
-    }
-    static constexpr long UNITS = (long)D::KK * D::NQ;
+    // fp32: as many CTAs as leave a thread about 100 registers; fp64: two
+    static constexpr int MIN_BLOCKS = sizeof(T) == 8 ? 2 : 20 / WARPS;
+    static constexpr int ROW = D::KK;  // Pairs
+    static constexpr size_t smem_bytes() { return (size_t)U * nslot<ROT>() * ROW * sizeof(Pair<T>); }
+    static constexpr int UNITS = D::KK * D::NQ;
+    static_assert(FftPlan<N>::SMEM * sizeof(cplx<T>) <= ROW * sizeof(Pair<T>), "exchange fits a row");
 };
 
 // Index of kept mode (c, ky', kz, kx') in the compact state / accumulator.
@@ -571,15 +575,14 @@ __global__ void __launch_bounds__(XPass<T, N, ROT>::THREADS, XPass<T, N, ROT>::M
     constexpr int RF0 = first_radix<N, false>(), RIL = last_radix<N, true>();
     constexpr int NH = N / 2 + 1;
     extern __shared__ __align__(16) unsigned char xsm[];
-    Pair<T>* stage = reinterpret_cast<Pair<T>*>(xsm);  // [u][f][kx']
+    Pair<T>* stage = reinterpret_cast<Pair<T>*>(xsm);  // rows [u][f][kx']
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int fw = warp % NF;                               // this warp's field slot
     const int sub = (warp / NF) * S + lane / TT, t = lane % TT;  // this sequence's unit in the CTA
-    cplx<T>* sm = reinterpret_cast<cplx<T>*>(xsm + X::stage_bytes()) +
-                  (size_t)(warp * S + lane / TT) * FftPlan<N>::SMEM;
-    const long unit = (long)blockIdx.x * U + sub;
+    cplx<T>* sm = reinterpret_cast<cplx<T>*>(stage + ((size_t)sub * NF + fw) * KK);
+    const int unit = blockIdx.x * U + sub;
     const bool active = unit < X::UNITS;
-    const int q = (int)(unit % D::NQ), kyi = (int)(unit / D::NQ);
+    const int q = unit % D::NQ, kyi = unit / D::NQ;
     const int kb = spec_base<N>(t), xb = phys_base<N>(t);
     const StepParams<T> p = *P;
     // thread 0: the CTA's compact state (and accumulator) rows into L2 while the forward
@@ -587,9 +590,9 @@ __global__ void __launch_bounds__(XPass<T, N, ROT>::THREADS, XPass<T, N, ROT>::M
     if (threadIdx.x == 0) {
         constexpr size_t CS = (size_t)KK * D::KZ * KK;  // one component
         for (int s = 0; s < U; ++s) {
-            const long us = (long)blockIdx.x * U + s;
+            const int us = blockIdx.x * U + s;
             if (us >= X::UNITS) break;
-            const int qs = (int)(us % D::NQ), kyis = (int)(us / D::NQ);
+            const int qs = us % D::NQ, kyis = us / D::NQ;
             const int nkz = D::KZ - 2 * qs < 2 ? D::KZ - 2 * qs : 2;
             if (nkz <= 0) continue;
             const size_t e0 = compact_idx<N>(0, kyis, 2 * qs, 0);
@@ -606,7 +609,31 @@ __global__ void __launch_bounds__(XPass<T, N, ROT>::THREADS, XPass<T, N, ROT>::M
         return stage[((size_t)s * NF + f) * KK + kxi];
     };
 
-    // forward along x of the products, kept kx into the staging buffer
+    // Element e of the CTA's columns: kept kx' = e % KK (fastest: the compact state and
+    // accumulator rows are read and written contiguously) of kz column e / KK = 2 s + h.
+    constexpr int TOT = U * 2 * KK;
+    constexpr size_t CS = (size_t)KK * D::KZ * KK;  // one component
+    struct Mode {
+        cplx<T> u[3], c[3];
+    };
+    // state and accumulator of element e, loaded one element ahead of the update
+    auto load_mode = [&](int e, Mode& md) {
+        const int col = e / KK, kxi = e - col * KK, us = blockIdx.x * U + (col >> 1);
+        const int qs = us % D::NQ, kyis = us / D::NQ, kzi = 2 * qs + (col & 1);
+        if (e < TOT && us < X::UNITS && kzi < D::KZ) {
+            const size_t o = compact_idx<N>(0, kyis, kzi, kxi);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                md.u[c] = u0[c * CS + o];
+                if (STAGE > 0) md.c[c] = acc[c * CS + o];
+            }
+        }
+    };
+    Mode nxt;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) nxt.u[c] = nxt.c[c] = mk<T>(0, 0);
+
+    // forward along x of the products, kept kx into the row
     if constexpr (STAGE >= 0) {
         if (fw < NFW) {
             const int f = fw;
@@ -618,22 +645,26 @@ __global__ void __launch_bounds__(XPass<T, N, ROT>::THREADS, XPass<T, N, ROT>::M
                     v[g * RF0 + m] = active ? Bs[spec_idx<N, ROT>(in_pos<N, RF0>(xb, g, m), f, kyi, q)]
                                             : pzero<T>();
             seq_fft<N, false, true>(v, sm, t, tw);
+            __syncwarp();  // the row held the exchange
             for_slots([&](auto mc) {
                 constexpr int M = decltype(mc)::value;
                 slot_store<N, M>(kb, [&](int k) { st_at(sub, f, kept_of_fft<N>(k)) = v[M]; });
             });
         }
+        load_mode(threadIdx.x, nxt);
         __syncthreads();
+    } else {
+        load_mode(threadIdx.x, nxt);
     }
 
-    // every kept kx of the CTA's columns, one kz column at a time (kx' fastest: the compact
-    // state and accumulator rows are read and written contiguously): update and next inputs
-#pragma unroll 2
-    for (int e = threadIdx.x; e < U * 2 * KK; e += X::THREADS) {
-        const int kxi = e % KK, sh = e / KK, s = sh >> 1, h = sh & 1;
-        const long us = (long)blockIdx.x * U + s;
+    // every kept kx of the CTA's columns: update and next inputs
+    for (int e = threadIdx.x; e < TOT; e += X::THREADS) {
+        const int col = e / KK, kxi = e - col * KK, s = col >> 1, h = col & 1;
+        const int us = blockIdx.x * U + s;
+        const Mode md = nxt;
+        load_mode(e + X::THREADS, nxt);
         if (us >= X::UNITS) continue;
-        const int qs = (int)(us % D::NQ), kyis = (int)(us / D::NQ);
+        const int qs = us % D::NQ, kyis = us / D::NQ;
         const int kzi = 2 * qs + h;
         cplx<T> out[6];
 #pragma unroll
@@ -642,8 +673,7 @@ __global__ void __launch_bounds__(XPass<T, N, ROT>::THREADS, XPass<T, N, ROT>::M
             const int kxs = kept_k<N>(kxi), kys = kept_k<N>(kyis);
             const T kx = (T)kxs, ky = (T)kys, kz = (T)kzi, k2 = kx * kx + ky * ky + kz * kz;
             const size_t o = compact_idx<N>(0, kyis, kzi, kxi);
-            constexpr size_t CS = (size_t)D::KK * D::KZ * D::KK;  // one component
-            cplx<T> a = u0[o], b = u0[CS + o], c = u0[2 * CS + o];
+            cplx<T> a = md.u[0], b = md.u[1], c = md.u[2];
             if constexpr (STAGE >= 0) {
                 cplx<T> F[NFW];
 #pragma unroll
@@ -673,9 +703,7 @@ __global__ void __launch_bounds__(XPass<T, N, ROT>::THREADS, XPass<T, N, ROT>::M
                 N2 = axpy(-kz, d, N2);
                 const IFac<T> fac = if_factors(tab, NH, kxs < 0 ? -kxs : kxs,
                                                kys < 0 ? -kys : kys, kzi, k2, p);
-                cplx<T> Ca = STAGE > 0 ? acc[o] : mk<T>(0, 0);
-                cplx<T> Cb = STAGE > 0 ? acc[CS + o] : mk<T>(0, 0);
-                cplx<T> Cc = STAGE > 0 ? acc[2 * CS + o] : mk<T>(0, 0);
+                cplx<T> Ca = md.c[0], Cb = md.c[1], Cc = md.c[2];  // zero at stage 0
                 constexpr int SG = STAGE < 0 ? 0 : STAGE;
                 a = lawson_stage<T, SG>(p.dt, fac, N0, a, Ca);
                 b = lawson_stage<T, SG>(p.dt, fac, N1, b, Cb);
@@ -723,6 +751,7 @@ __global__ void __launch_bounds__(XPass<T, N, ROT>::THREADS, XPass<T, N, ROT>::M
             auto hi = [&](int k) { return st_at(sub, f, k - N + KK); };
             v[M] = slot_value<N, M>(kb, lo, hi, pzero<T>());
         });
+        __syncwarp();  // the row is in registers: it takes the exchange
         seq_fft<N, true, true>(v, sm, t, tw);
         if (active) {
 #pragma unroll
