@@ -253,18 +253,32 @@ __device__ __forceinline__ void stage_weights(unsigned char* sW, const __nv_bflo
     }
 }
 
-// Forward epilogue of a hidden layer: row p of Z (64 columns) -> GELU -> bf16 hidden tile.
+// Forward epilogue of a hidden layer: 16 columns c0 .. of row p of Z -> GELU -> bf16 hidden tile.
 __device__ __forceinline__ void epi_forward(uint32_t tbase, uint32_t zcol, unsigned char* sHt,
-                                            int p, int warp) {
-#pragma unroll 1
-    for (int c = 0; c < kH; c += 8) {
-        float z[8];
-        tc::tmem_ld8(tc::tmem_at(tbase, 32 * warp, zcol + c), z);
-        tc::tmem_wait_ld();
+                                            int p, int quad, int c0) {
+    float z[16];
+    tc::tmem_ld16(tc::tmem_at(tbase, 32 * quad, zcol + c0), z);
+    tc::tmem_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 8; ++i) z[i] = gelu(z[i]);
-        st_row8(sHt, p, c, kK, z);
+    for (int i = 0; i < 16; ++i) z[i] = gelu(z[i]);
+    st_row8(sHt, p, c0, kK, z);
+    st_row8(sHt, p, c0 + 8, kK, z + 8);
+}
+
+// Backward epilogue: 16 columns of the layer's data gradient times GELU' of its pre-activation.
+__device__ __forceinline__ void epi_backward(uint32_t tbase, uint32_t dcol, uint32_t zcol,
+                                             unsigned char* sDZ, int p, int quad, int c0) {
+    float dh[16], z[16];
+    tc::tmem_ld16(tc::tmem_at(tbase, 32 * quad, dcol + c0), dh);
+    tc::tmem_ld16(tc::tmem_at(tbase, 32 * quad, zcol + c0), z);
+    tc::tmem_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        float h;
+        dh[i] *= gelu_d(z[i], h);
     }
+    st_row8(sDZ, p, c0, kH, dh);
+    st_row8(sDZ, p, c0 + 8, kH, dh + 8);
 }
 
 // Sum over a warp of 8 values per lane; lanes with (lane & 3) == 0 return the sum of column
@@ -308,7 +322,8 @@ struct TrainSmem {
     static constexpr int ST = DZ + kTile * kH * 2;               // stencil floats
     static constexpr int W4 = ST + kStencil * 4;                 // w4 fp32 [80]
     static constexpr int DW4 = W4 + kK * 4;                      // dw4 partials fp32 [4][80]
-    static constexpr int BYTES = DW4 + 4 * kK * 4;
+    static constexpr int YP = DW4 + 4 * kK * 4;                  // output partials fp32 [4][128]
+    static constexpr int BYTES = YP + 4 * kTile * 4;
 };
 static_assert(TrainSmem::W4 % 16 == 0, "alignment");
 // A CTA's row of the partials buffer: the 15440 gradient sums, then its loss sum.
@@ -319,11 +334,21 @@ constexpr uint32_t kTrainCols = 512;
 
 // One CTA per SM; each CTA runs forward + backward over its share of the batch's tiles and
 // writes its summed gradient to partials[blockIdx.x][15440].
-__global__ void __launch_bounds__(128, 1)
+// Sixteen warps: warps w, w + 4, w + 8, w + 12 serve the TMEM lanes (points) 32 (w % 4) .. + 31
+// and 16 of the 64 hidden columns each.  The tensor pipe works a few percent of a tile's time;
+// the tile is bound by its GELU epilogues (two MUFU and about twenty fp32 operations for each
+// of some 450 values per point), which four warps, one per scheduler, ran at the latency of
+// their dependency chains.  65536 points: 69.5 -> 55.8 us per
+// launch.
+constexpr int kTrainThreads = 512;
+constexpr int kTrainGroups = kTrainThreads / kTile;  // column groups of 16
+
+__global__ void __launch_bounds__(kTrainThreads, 1)
     k_train(const float* __restrict__ bank, int n, int count, const __nv_bfloat16* __restrict__ wb,
             const float* __restrict__ params, const Consts* __restrict__ ccp,
             const int* __restrict__ step_dev, int64_t step_override, uint64_t seed, int ntiles,
             float inv_batch, float* __restrict__ partials, int* __restrict__ err) {
+    static_assert(kTrainGroups == 4 && kH == 16 * kTrainGroups, "16 columns per group");
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tslot;
@@ -336,27 +361,31 @@ __global__ void __launch_bounds__(128, 1)
     float* sSt = reinterpret_cast<float*>(smem + TrainSmem::ST);
     float* sW4 = reinterpret_cast<float*>(smem + TrainSmem::W4);
     float* sDW4 = reinterpret_cast<float*>(smem + TrainSmem::DW4);
+    float* sYP = reinterpret_cast<float*>(smem + TrainSmem::YP);
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int quad = warp & 3, cg = warp >> 2;  // TMEM lane quadrant, column group
+    const int p = 32 * quad + lane;             // this thread's point in the tile
+    const int c0 = 16 * cg;                     // its hidden columns c0 .. c0 + 15
     const Consts cc = *ccp;
     const int64_t step = step_override >= 0 ? step_override : (int64_t)*step_dev;
 
     // the stencil and target of the CTA's next tile are loaded while the current one computes
     // (the first tile's while the weights are staged)
-    float nxt[stencil_per_thread<128>()];
+    float nxt[stencil_per_thread<kTrainThreads>()];
     float nxt_target = 0.f;
     auto load_tile = [&](int tl) {
         const TilePick pk = pick_tile(seed, step, tl, count, n);
         const int y0 = pk.seg * kTile;
         const float* snap = bank + (size_t)pk.snap * 4 * n * n;
-        nxt_target = snap[3 * (size_t)n * n + (size_t)pk.row * n + y0 + t];
-        stencil_load<128>(nxt, snap, (size_t)n * n, n, n, pk.row, y0);
+        nxt_target = snap[3 * (size_t)n * n + (size_t)pk.row * n + y0 + p];
+        stencil_load<kTrainThreads>(nxt, snap, (size_t)n * n, n, n, pk.row, y0);
     };
     if (blockIdx.x < ntiles) load_tile(blockIdx.x);
-    stage_weights<128>(sW, wb);
+    stage_weights<kTrainThreads>(sW, wb);
     if (t < kK) sW4[t] = params[kLayers * kWsz + t];
-    for (int i = t; i < 4 * kK; i += blockDim.x) sDW4[i] = 0.f;  // one row per warp
-    init_hidden_bias(sH1, t);
-    init_hidden_bias(sH2, t);
+    for (int i = t; i < 4 * kK; i += blockDim.x) sDW4[i] = 0.f;  // one row per lane quadrant
+    if (cg == 0) init_hidden_bias(sH1, p);
+    if (cg == 1) init_hidden_bias(sH2, p);
     if (t == 0) {
         tc::mbar_init(&bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -372,11 +401,15 @@ __global__ void __launch_bounds__(128, 1)
     bool ok = true, first = true;
     float loss = 0.f;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        stencil_store<128>(sSt, nxt, cc);
+        stencil_store<kTrainThreads>(sSt, nxt, cc);
         const float target = nxt_target * cc.inv_outscale;
         if (tile + (int)gridDim.x < ntiles) load_tile(tile + gridDim.x);
         __syncthreads();
-        build_x(sX, sSt, t);
+        // ten feature groups of 8 over the four column groups
+        if (cg == 0) build_x<0, 3>(sX, sSt, p);
+        else if (cg == 1) build_x<3, 6>(sX, sSt, p);
+        else if (cg == 2) build_x<6, 8>(sX, sSt, p);
+        else build_x<8, kK / 8>(sX, sSt, p);
 
         // ---- forward: three tensor-core layers
         sync_for_mma();
@@ -385,14 +418,14 @@ __global__ void __launch_bounds__(128, 1)
             tc::mma_commit(&bar);
         }
         if (!(ok = wait_mma(&bar, phase))) break;
-        epi_forward(tb, kZ1, sH1, t, warp);
+        epi_forward(tb, kZ1, sH1, p, quad, c0);
         sync_for_mma();
         if (t == 0) {
             issue(tb + kZ2, aH1, 0, kK, aW2, 0, kK, 128, kH, kK / 16, false);
             tc::mma_commit(&bar);
         }
         if (!(ok = wait_mma(&bar, phase))) break;
-        epi_forward(tb, kZ2, sH2, t, warp);
+        epi_forward(tb, kZ2, sH2, p, quad, c0);
         sync_for_mma();
         if (t == 0) {
             issue(tb + kZ3, aH2, 0, kK, aW3, 0, kK, 128, kH, kK / 16, false);
@@ -401,38 +434,45 @@ __global__ void __launch_bounds__(128, 1)
         if (!(ok = wait_mma(&bar, phase))) break;
 
         // ---- output layer, loss, and the layer-3 gradient
-        float y = sW4[kBiasH];
-#pragma unroll 1
-        for (int c = 0; c < kH; c += 8) {
-            float z[8];
-            tc::tmem_ld8(tc::tmem_at(tb, 32 * warp, kZ3 + c), z);
+        float h3[16], g3[16];  // activations and GELU' of layer 3
+        {
+            float z[16];
+            tc::tmem_ld16(tc::tmem_at(tb, 32 * quad, kZ3 + c0), z);
             tc::tmem_wait_ld();
+            float y = 0.f;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) y += gelu(z[i]) * sW4[c + i];
+            for (int i = 0; i < 16; ++i) {
+                g3[i] = gelu_d(z[i], h3[i]);
+                y += h3[i] * sW4[c0 + i];
+            }
+            sYP[cg * kTile + p] = y;
         }
+        __syncthreads();
+        const float y = (((sW4[kBiasH] + sYP[p]) + sYP[kTile + p]) + sYP[2 * kTile + p]) +
+                        sYP[3 * kTile + p];
         const float r = y - target;
         const float dy = 2.f * r * inv_batch;
-        loss += r * r;
-#pragma unroll 1
-        for (int c = 0; c < kH; c += 8) {
-            float z[8], dz[8];
-            tc::tmem_ld8(tc::tmem_at(tb, 32 * warp, kZ3 + c), z);
-            tc::tmem_wait_ld();
+        if (cg == 0) loss += r * r;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                float h;
-                const float d = gelu_d(z[i], h);
-                dz[i] = dy * sW4[c + i] * d;
-                z[i] = dy * h;  // output-layer weight gradient contribution
-            }
-            st_row8(sDZ, t, c, kH, dz);
-            const int col = warp_sum8(z, lane);
-            // lanes 0, 4, .., 28 hold distinct columns: this warp's row, no atomics
-            if ((lane & 3) == 0) sDW4[warp * kK + c + col] += z[0];
+        for (int i = 0; i < 16; ++i) {
+            g3[i] = dy * sW4[c0 + i] * g3[i];
+            h3[i] = dy * h3[i];  // output-layer weight gradient contribution
         }
-        {
+        st_row8(sDZ, p, c0, kH, g3);
+        st_row8(sDZ, p, c0 + 8, kH, g3 + 8);
+#pragma unroll
+        for (int c = 0; c < 16; c += 8) {
+            float z[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) z[i] = h3[c + i];
+            const int col = warp_sum8(z, lane);
+            // lanes 0, 4, .., 28 hold distinct columns: this warp's share of its quadrant's
+            // row, no atomics
+            if ((lane & 3) == 0) sDW4[quad * kK + c0 + c + col] += z[0];
+        }
+        if (cg == 0) {
             const float sdy = warp_sum(dy);
-            if (lane == 0) sDW4[warp * kK + kBiasH] += sdy;
+            if (lane == 0) sDW4[quad * kK + kBiasH] += sdy;
         }
 
         // ---- backward through layers 3, 2, 1
@@ -443,19 +483,7 @@ __global__ void __launch_bounds__(128, 1)
             tc::mma_commit(&bar);
         }
         if (!(ok = wait_mma(&bar, phase))) break;
-#pragma unroll 1
-        for (int c = 0; c < kH; c += 8) {
-            float dh[8], z[8];
-            tc::tmem_ld8(tc::tmem_at(tb, 32 * warp, kDH + c), dh);
-            tc::tmem_ld8(tc::tmem_at(tb, 32 * warp, kZ2 + c), z);
-            tc::tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                float h;
-                dh[i] *= gelu_d(z[i], h);
-            }
-            st_row8(sDZ, t, c, kH, dh);
-        }
+        epi_backward(tb, kDH, kZ2, sDZ, p, quad, c0);
         sync_for_mma();
         if (t == 0) {
             issue(tb + kGW2, aDZ, 1, kH, aH1, 1, kK, 64, kK, kTile / 16, !first);
@@ -463,19 +491,7 @@ __global__ void __launch_bounds__(128, 1)
             tc::mma_commit(&bar);
         }
         if (!(ok = wait_mma(&bar, phase))) break;
-#pragma unroll 1
-        for (int c = 0; c < kH; c += 8) {
-            float dh[8], z[8];
-            tc::tmem_ld8(tc::tmem_at(tb, 32 * warp, kDH + c), dh);
-            tc::tmem_ld8(tc::tmem_at(tb, 32 * warp, kZ1 + c), z);
-            tc::tmem_wait_ld();
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                float h;
-                dh[i] *= gelu_d(z[i], h);
-            }
-            st_row8(sDZ, t, c, kH, dh);
-        }
+        epi_backward(tb, kDH, kZ1, sDZ, p, quad, c0);
         sync_for_mma();
         if (t == 0) {
             issue(tb + kGW1, aDZ, 1, kH, aX, 1, kK, 64, kK, kTile / 16, !first);
@@ -490,19 +506,19 @@ __global__ void __launch_bounds__(128, 1)
         const uint32_t gw[3] = {kGW1, kGW2, kGW3};
         for (int l = 0; l < kLayers; ++l) {
 #pragma unroll 1
-            for (int c = 0; c < kK; c += 8) {
+            for (int c = 8 * cg; c < kK; c += 8 * kTrainGroups) {
                 float v[8];
-                tc::tmem_ld8(tc::tmem_at(tb, 32 * warp, gw[l] + c), v);
+                tc::tmem_ld8(tc::tmem_at(tb, 32 * quad, gw[l] + c), v);
                 tc::tmem_wait_ld();
                 if (lane < 16) {
-                    float* dst = out + l * kWsz + (16 * warp + lane) * kK + c;
+                    float* dst = out + l * kWsz + (16 * quad + lane) * kK + c;
 #pragma unroll
                     for (int i = 0; i < 8; ++i) dst[i] = v[i];
                 }
             }
         }
         loss = warp_sum(loss);
-        if (lane == 0) sLoss[warp] = loss;
+        if (cg == 0 && lane == 0) sLoss[quad] = loss;
         __syncthreads();
         // fixed summation orders throughout: the gradient and loss are bit-reproducible
         if (t < kK) out[kLayers * kWsz + t] = ((sDW4[t] + sDW4[kK + t]) + sDW4[2 * kK + t]) +
@@ -522,32 +538,11 @@ struct AdamCfg {
     int total, warmup;
 };
 
-// Sums the CTAs' partial rows in order; thread kNParam also records the step's loss and (when
-// `advance`) moves the step counter on — one thread reads and writes it.
-__global__ void k_grad_reduce(const float* __restrict__ partials, int nblk, float* __restrict__ grad,
-                              int* __restrict__ step_dev, int64_t step_override,
-                              float* __restrict__ loss_ring, int advance) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j > kNParam) return;
-    float s = 0.f;
-    for (int b = 0; b < nblk; ++b) s += partials[(size_t)b * kPartStride + j];
-    if (j < kNParam) {
-        grad[j] = s;
-        return;
-    }
-    const int64_t step = step_override >= 0 ? step_override : (int64_t)*step_dev;
-    loss_ring[step & (kLossRing - 1)] = s;
-    if (advance) *step_dev = (int)step + 1;
-}
-
-// Adam (Kingma and Ba) with a linear warm-up and cosine decay of the learning rate; step_dev
-// holds the 1-based step number of this update.
-__global__ void k_adam(float* __restrict__ params, float* __restrict__ m, float* __restrict__ v,
-                       const float* __restrict__ grad, __nv_bfloat16* __restrict__ wb,
-                       const int* __restrict__ step_dev, AdamCfg cfg) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= kNParam) return;
-    const int t = *step_dev;
+// Adam (Kingma and Ba) with a linear warm-up and cosine decay of the learning rate; t is the
+// 1-based step number of this update.
+__device__ __forceinline__ void adam_update(int j, float g, int t, const AdamCfg& cfg,
+                                            float* __restrict__ params, float* __restrict__ m,
+                                            float* __restrict__ v, __nv_bfloat16* __restrict__ wb) {
     float lr;
     if (cfg.warmup > 0 && t <= cfg.warmup) {
         lr = cfg.lr * (float)t / (float)cfg.warmup;
@@ -556,7 +551,6 @@ __global__ void k_adam(float* __restrict__ params, float* __restrict__ m, float*
         const float x = fminf((float)(t - cfg.warmup) / span, 1.f);
         lr = cfg.lr_min + 0.5f * (cfg.lr - cfg.lr_min) * (1.f + cospif(x));
     }
-    const float g = grad[j];
     const float mj = cfg.b1 * m[j] + (1.f - cfg.b1) * g;
     const float vj = cfg.b2 * v[j] + (1.f - cfg.b2) * g * g;
     m[j] = mj;
@@ -566,6 +560,58 @@ __global__ void k_adam(float* __restrict__ params, float* __restrict__ m, float*
     const float p = params[j] - lr * mh / (sqrtf(vh) + cfg.eps);
     params[j] = p;
     if (j < kLayers * kWsz) wb[wb_index(j)] = __float2bfloat16_rn(p);
+}
+
+// Sums the CTAs' partial rows: 32 parameters per CTA, warp g sums rows g, g + 8, .. of them (one
+// 128-byte access each) and the eight sums are added in order, so the gradient is
+// bit-reproducible.  (One thread per parameter over all the rows was a chain of 148 loads in 61
+// CTAs: 10.1 us, and the update 5.3 us after it; one launch of 8.4 us now, cold.)  The column kNParam is the step's loss.  ADAM: the same thread then updates
+// its parameter; `advance` moves the step counter on once every CTA has read it (the last CTA to
+// finish, by `ticket`).
+constexpr int kReduceRows = 8;
+template <bool ADAM>
+__global__ void __launch_bounds__(32 * kReduceRows)
+    k_grad_reduce(const float* __restrict__ partials, int nblk, float* __restrict__ grad,
+                  int* __restrict__ step_dev, int64_t step_override, float* __restrict__ loss_ring,
+                  int advance, unsigned* __restrict__ ticket, float* __restrict__ params,
+                  float* __restrict__ m, float* __restrict__ v, __nv_bfloat16* __restrict__ wb,
+                  AdamCfg cfg) {
+    __shared__ float part[kReduceRows][32];
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const int j = blockIdx.x * 32 + lane;
+    const int64_t step = step_override >= 0 ? step_override : (int64_t)*step_dev;
+    float s = 0.f;
+    if (j <= kNParam) {
+#pragma unroll 8
+        for (int b = g; b < nblk; b += kReduceRows) s += partials[(size_t)b * kPartStride + j];
+    }
+    part[g][lane] = s;
+    __syncthreads();
+    if (g == 0 && j <= kNParam) {
+        s = part[0][lane];
+#pragma unroll
+        for (int q = 1; q < kReduceRows; ++q) s += part[q][lane];
+        if (j < kNParam) {
+            grad[j] = s;
+            if (ADAM) adam_update(j, s, (int)step + 1, cfg, params, m, v, wb);
+        } else {
+            loss_ring[step & (kLossRing - 1)] = s;
+        }
+    }
+    if (advance && threadIdx.x == 0) {
+        // this CTA's step was read before the barrier above
+        if (atomicAdd(ticket, 1u) == gridDim.x - 1) {
+            *step_dev = (int)step + 1;
+            *ticket = 0;
+        }
+    }
+}
+
+__global__ void k_adam(float* __restrict__ params, float* __restrict__ m, float* __restrict__ v,
+                       const float* __restrict__ grad, __nv_bfloat16* __restrict__ wb,
+                       const int* __restrict__ step_dev, AdamCfg cfg) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < kNParam) adam_update(j, grad[j], *step_dev, cfg, params, m, v, wb);
 }
 
 __global__ void k_to_bf16(const float* __restrict__ params, __nv_bfloat16* __restrict__ wb) {
@@ -791,6 +837,7 @@ struct sp_closure {
     float* loss = nullptr;
     __nv_bfloat16* wb = nullptr;
     int* step_dev = nullptr;
+    unsigned* ticket = nullptr;  // CTAs of the gradient reduction that have finished
     int* err = nullptr;
     Consts* consts_dev = nullptr;
     float* shell_gain = nullptr;  // per-shell gain of the closure term in the coarse step
@@ -842,20 +889,21 @@ int launch_train_step(sp_closure* c, int ntiles, uint64_t seed, int64_t step_ove
                       bool advance, bool adam, cudaStream_t st) {
     const int grid = ntiles < c->sms ? ntiles : c->sms;
     const float inv_batch = 1.f / ((float)ntiles * (float)kTile);
-    k_train<<<grid, 128, TrainSmem::BYTES, st>>>(c->bank, c->n, c->count, c->wb, c->params,
+    k_train<<<grid, kTrainThreads, TrainSmem::BYTES, st>>>(c->bank, c->n, c->count, c->wb, c->params,
                                                  c->consts_dev, c->step_dev, step_override, seed,
                                                  ntiles, inv_batch, c->partials, c->err);
     CL_CUDA(cudaGetLastError());
-    k_grad_reduce<<<(kNParam + 1 + 255) / 256, 256, 0, st>>>(
-        c->partials, grid, c->grad, c->step_dev, step_override, c->loss, advance ? 1 : 0);
+    const int rgrid = (kNParam + 1 + 31) / 32;
+    if (adam)
+        k_grad_reduce<true><<<rgrid, 32 * kReduceRows, 0, st>>>(
+            c->partials, grid, c->grad, c->step_dev, step_override, c->loss, advance ? 1 : 0,
+            c->ticket, c->params, c->adam_m, c->adam_v, c->wb, c->adam);
+    else
+        k_grad_reduce<false><<<rgrid, 32 * kReduceRows, 0, st>>>(
+            c->partials, grid, c->grad, c->step_dev, step_override, c->loss, advance ? 1 : 0,
+            c->ticket, c->params, c->adam_m, c->adam_v, c->wb, c->adam);
     CL_CUDA(cudaGetLastError());
     c->launches += 2;
-    if (adam) {
-        k_adam<<<(kNParam + 255) / 256, 256, 0, st>>>(c->params, c->adam_m, c->adam_v, c->grad,
-                                                      c->wb, c->step_dev, c->adam);
-        CL_CUDA(cudaGetLastError());
-        c->launches += 1;
-    }
     return SP_OK;
 }
 
@@ -937,6 +985,7 @@ sp_closure* sp_closure_create(int n, int capacity, int* status) {
                cudaMalloc(&c->loss, kLossRing * sizeof(float)) == cudaSuccess &&
                cudaMalloc(&c->wb, kLayers * kWsz * sizeof(__nv_bfloat16)) == cudaSuccess &&
                cudaMalloc(&c->step_dev, sizeof(int)) == cudaSuccess &&
+               cudaMalloc(&c->ticket, sizeof(unsigned)) == cudaSuccess &&
                cudaMalloc(&c->err, sizeof(int)) == cudaSuccess &&
                cudaMalloc(&c->consts_dev, sizeof(Consts)) == cudaSuccess &&
                cudaMalloc(&c->spec, 4 * (size_t)c->fsc * sizeof(cplx<float>)) == cudaSuccess;
@@ -950,6 +999,7 @@ sp_closure* sp_closure_create(int n, int capacity, int* status) {
                cudaMemset(c->loss, 0, kLossRing * sizeof(float)) == cudaSuccess &&
                cudaMemset(c->wb, 0, kLayers * kWsz * sizeof(__nv_bfloat16)) == cudaSuccess &&
                cudaMemset(c->step_dev, 0, sizeof(int)) == cudaSuccess &&
+               cudaMemset(c->ticket, 0, sizeof(unsigned)) == cudaSuccess &&
                cudaMemset(c->err, 0, sizeof(int)) == cudaSuccess;
     if (!okz) return fail_create("initialisation failed");
     {
@@ -994,7 +1044,7 @@ void sp_closure_destroy(sp_closure* c) {
     if (c->have_plan) cufftDestroy(c->plan);
     for (void* p : {(void*)c->bank, (void*)c->params, (void*)c->adam_m, (void*)c->adam_v,
                     (void*)c->grad, (void*)c->partials, (void*)c->loss, (void*)c->wb,
-                    (void*)c->step_dev, (void*)c->err, (void*)c->consts_dev, (void*)c->spec,
+                    (void*)c->step_dev, (void*)c->ticket, (void*)c->err, (void*)c->consts_dev, (void*)c->spec,
                     (void*)c->shell_gain, c->plan_ws})
         if (p) cudaFree(p);
     delete c;
@@ -1164,7 +1214,7 @@ int sp_closure_train(sp_closure* c, int steps, int batch_tiles, uint64_t seed, v
         }
         for (; done + kChunk <= steps; done += kChunk) {
             CL_CUDA(cudaGraphLaunch(c->exec, st));
-            c->launches += 3 * kChunk;
+            c->launches += 2 * kChunk;
         }
     }
     for (; done < steps; ++done) {
