@@ -274,12 +274,12 @@ __global__ void __launch_bounds__(RowPairs<N>::THREADS) k_row_max(const Pair<T>*
             bv = max(bv, __shfl_down_sync(0xffffffffu, bv, o));
         }
         if ((threadIdx.x & 31) == 0) {
-            atomicMax(umax + 0, bu);
-            atomicMax(umax + 1, bv);
+            raise_max(umax + 0, bu);
+            raise_max(umax + 1, bv);
         }
     } else {  // tiny grids: a partial warp, no shuffles
-        atomicMax(umax + 0, bu);
-        atomicMax(umax + 1, bv);
+        raise_max(umax + 0, bu);
+        raise_max(umax + 1, bv);
     }
 }
 

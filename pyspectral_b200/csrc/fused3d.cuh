@@ -460,9 +460,9 @@ __global__ void __launch_bounds__(z_threads<T>()) k3_z(Pair<T>* __restrict__ Bp,
             bw = max(bw, __shfl_down_sync(0xffffffffu, bw, o));
         }
         if ((threadIdx.x & 31) == 0) {
-            atomicMax(umax + 0, bu);
-            atomicMax(umax + 1, bv);
-            atomicMax(umax + 2, bw);
+            raise_max(umax + 0, bu);
+            raise_max(umax + 1, bv);
+            raise_max(umax + 2, bw);
         }
     }
 
