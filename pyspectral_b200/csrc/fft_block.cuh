@@ -183,6 +183,50 @@ __device__ __forceinline__ void dft16(E* x) {
     }
 }
 
+// dft16<+1> of inputs with x[7] = 0 and x[15] = c r (a product of a real and a complex value),
+// x[15] holding the rounded product: where fx (fy) is set, the sums that take the product's real
+// (imaginary) part are fused multiply-adds of the unrounded product.
+template <typename C, typename R>
+__device__ __forceinline__ void dft16_fused15(C* x, R c, C r, bool fx, bool fy) {
+    // the product as m q: (c, r) where fused, (1, rounded) where not
+    const R mx = fx ? c : (R)1, qx = fx ? r.x : x[15].x;
+    const R my = fy ? c : (R)1, qy = fy ? r.y : x[15].y;
+    const C a = eadd(x[3], x[11]), b = esub(x[3], x[11]);
+    C y[16];
+#pragma unroll
+    for (int n2 = 0; n2 < 3; ++n2) {
+        C p = x[n2], q = x[4 + n2], u = x[8 + n2], w = x[12 + n2];
+        dft4<1>(p, q, u, w);
+        y[n2 * 4 + 0] = p;
+        y[n2 * 4 + 1] = q;
+        y[n2 * 4 + 2] = u;
+        y[n2 * 4 + 3] = w;
+    }
+    // a + x15, b - i x15, a - x15, b + i x15
+    y[12] = mk<R>(fma(mx, qx, a.x), fma(my, qy, a.y));
+    y[13] = mk<R>(fma(my, qy, b.x), fma(-mx, qx, b.y));
+    y[14] = mk<R>(fma(-mx, qx, a.x), fma(-my, qy, a.y));
+    y[15] = mk<R>(fma(-my, qy, b.x), fma(mx, qx, b.y));
+    y[5] = rot16<1, 1>(y[5]);
+    y[6] = rot16<1, 2>(y[6]);
+    y[7] = rot16<1, 3>(y[7]);
+    y[9] = rot16<1, 2>(y[9]);
+    y[10] = rot16<1, 4>(y[10]);
+    y[11] = rot16<1, 6>(y[11]);
+    y[13] = rot16<1, 3>(y[13]);
+    y[14] = rot16<1, 6>(y[14]);
+    y[15] = rot16<1, 9>(y[15]);
+#pragma unroll
+    for (int k1 = 0; k1 < 4; ++k1) {
+        C p = y[k1], q = y[4 + k1], u = y[8 + k1], w = y[12 + k1];
+        dft4<1>(p, q, u, w);
+        x[k1 + 0] = p;
+        x[k1 + 4] = q;
+        x[k1 + 8] = u;
+        x[k1 + 12] = w;
+    }
+}
+
 template <int R, int DIR, typename E>
 __device__ __forceinline__ void dftR(E* x) {
     if constexpr (R == 2) dft2<DIR>(x);
@@ -389,15 +433,17 @@ __device__ __forceinline__ void pass_compute_h(E (&v)[16], int t, const C* __res
 // radix(INV, 0)); on exit v holds the output at in_pos with the last pass's radix.  `sm` is this
 // sequence's padded shared buffer; every thread of the CTA must call (barriers inside).  TWINV
 // picks the table blocks: a forward transform whose passes have the inverse's radices and
-// strides (N = 16^k) may read the inverse blocks, conjugated.
-template <int N, bool INV, bool WARP = false, bool TWINV = INV, typename E, typename C>
+// strides (N = 16^k) may read the inverse blocks, conjugated.  FIRST = false: the caller has done
+// the first pass's DFTs.
+template <int N, bool INV, bool WARP = false, bool TWINV = INV, bool FIRST = true, typename E,
+          typename C>
 __device__ __forceinline__ void block_fft(E (&v)[16], E* sm, int t, const C* __restrict__ tw) {
     using P = FftPlan<N>;
     static_assert(!WARP || P::T <= 32, "a warp-synchronised transform fits in one warp");
     constexpr int DIR = INV ? 1 : -1;
     static_assert(TWINV == INV || P::R0 == 1, "shared blocks need equal pass structures");
     constexpr int R0 = P::radix(INV, 0), S0 = P::stride(INV, 0);
-    pass_compute<N, R0, S0, DIR>(v, t, tw);  // S0 = 1: no twiddles
+    if constexpr (FIRST) pass_compute<N, R0, S0, DIR>(v, t, tw);  // S0 = 1: no twiddles
     if constexpr (P::NP > 1) {
         constexpr int R1 = P::radix(INV, 1), S1 = P::stride(INV, 1);
         pass_store<N, R0, S0>(v, sm, t);
@@ -598,6 +644,22 @@ __device__ __forceinline__ void seq_fft(E (&v)[16], S* sm, int t, const C* __res
         else split_forward<N, WARP>(v, sm, split_role<N / 16>(t), tw);
     } else {
         half_fft<N, INV, WARP, INV>(v, sm, t, tw);
+    }
+}
+// The inverse of seq_fft on from the first pass: the caller has done the DFTs of its sixteen
+// inputs (dft16, radix 16 without twiddles in both forms).
+template <int N, typename E, typename C>
+__device__ __forceinline__ void seq_inverse_rest(E (&v)[16], E* sm, int t, const C* __restrict__ tw) {
+    static_assert(FftPlan<N>::radix(true, 0) == 16, "radix-16 first pass");
+    if constexpr (split_plan<N>()) {
+        using P = FftPlan<N>;
+        constexpr int H = P::T / 2;
+        const int r = split_role<P::T>(t), h = r / H;
+        block_fft<N / 2, true, false, true, false>(v, sm + h * FftPlan<N / 2>::SMEM, r - h * H, tw);
+        half_trade<P::T>(v, h);
+        radix2_half_group<1, 0>(v, tw_load<1>(tw + P::tw_offset(true, P::NP - 1), r));
+    } else {
+        block_fft<N, true, false, true, false>(v, sm, t, tw);
     }
 }
 template <int N>

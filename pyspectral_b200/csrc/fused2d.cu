@@ -231,7 +231,7 @@ cudaError_t col_stage(const ColArgs& a) {
         }
         using F = Fused2D<N, BX>;
         const int grid = (a.kc + F::B - 1) / F::B;
-        k_col_pass<T, N, STAGE, BX><<<dim3(grid, a.members), F::THREADS,
+        k_col_pass<T, N, STAGE, BX><<<dim3(grid, a.members), col_threads<N, STAGE, BX>(),
                                       F::template smem_bytes<Pair<T>>(), a.st>>>(
             (Pair<T>*)a.X, a.kc, (cplx<T>*)a.u0t, (cplx<T>*)a.acct, (const T*)a.tab,
             (const StepParams<T>*)a.P, (const cplx<T>*)a.tw, a.xs, a.us, a.ts);

@@ -408,18 +408,174 @@ __device__ __forceinline__ void col_pass_cols(Pair<T>* __restrict__ X, int kc,
     }
 }
 
+// products that are not to be fused into a following sum
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
+// Grids whose column pass gives each of a column's two sequences its own threads.  Above, the
+// streamed pass's prefetch buffer leaves no room for two exchange buffers, and it is faster than
+// this pass without the prefetch (2048^2 fp32 0.173 against 0.187 ms per step, 4096^2 0.651
+// against 0.833).
+template <int N>
+constexpr bool split_columns() { return N <= 1024; }
+
+// The column pass (stages 0..3) with 2 (n/16) threads per column: thread s n/16 + t transforms
+// sequence s of the pair (P, Q) forward and of (u, v) back, and updates the slots m = s (mod 2) of
+// its index k0 + m n/16; the values of the other sequence at these slots are traded with thread
+// (1 - s) n/16 + t through the exchange buffers, before and after the update.  The state and
+// accumulator of the thread's slots are loaded together before the first trade.
+// Against one thread per pair (col_pass_cols) a thread holds half the registers and issues half
+// the instructions: small grids are bound by one warp's chain of about 2600 instructions per SM,
+// large ones by the warps that registers leave resident.  One B200, per step: 64^2 fp64 45.5 -> 31
+// us, 256^2 fp64 49 -> 37 us, 512^2 fp32 54.7 -> 43.6 us; ensemble of 64 runs each at 128^2..1024^2
+// fp32 3.78 -> 3.53 ms.
+template <typename T, int N, int STAGE, int B, bool FUSE_U>
+__device__ __forceinline__ void col_pass_split(Pair<T>* __restrict__ X, int kc,
+                                               cplx<T>* __restrict__ u0t,
+                                               cplx<T>* __restrict__ acct,
+                                               const T* __restrict__ tab, const StepParams<T>& p,
+                                               const cplx<T>* __restrict__ tw, int ky0,
+                                               unsigned char* smem_raw) {
+    static_assert(STAGE >= 0, "the set-up pass has no forward transform");
+    constexpr int TT = N / 16;
+    constexpr int RF0 = first_radix<N, false>();
+    constexpr int RIL = last_radix<N, true>();
+    static_assert(first_radix<N, true>() == 16 && last_radix<N, false>() == 16,
+                  "slot m holds row index k0 + m n/16");
+    const int sub = threadIdx.x / (2 * TT), q = threadIdx.x % (2 * TT);
+    const int s = q / TT, t = q % TT;
+    cplx<T>* own = reinterpret_cast<cplx<T>*>(smem_raw) + (2 * sub + s) * FftPlan<N>::SMEM;
+    const cplx<T>* mate = reinterpret_cast<const cplx<T>*>(smem_raw) + (2 * sub + 1 - s) * FftPlan<N>::SMEM;
+    const int ky = ky0 + sub;
+    const bool active = ky < kc;
+    const int xb = phys_base<N>(t), k0 = spec_base<N>(t);
+    // this sequence of the column: element x is Xs[2 xidx(x, ky, kc)]
+    cplx<T>* Xs = reinterpret_cast<cplx<T>*>(X) + s;
+
+    cplx<T> v[16];
+#pragma unroll
+    for (int g = 0; g < 16 / RF0; ++g)
+#pragma unroll
+        for (int m = 0; m < RF0; ++m) {
+            const int x = in_pos<N, RF0>(xb, g, m);
+            v[g * RF0 + m] = active ? Xs[2 * xidx(x, ky, kc)] : mk<T>(0, 0);
+        }
+    seq_fft<N, false>(v, own, t, tw);
+
+    const T kyr = (T)ky;
+    constexpr int nh = N / 2 + 1;
+    auto row_of = [&](int j) { return k0 + (2 * j + s) * TT; };  // this thread's slot 2 j + s
+    auto kept = [&](int i) {
+        const int kxi = signed_k(i, N);
+        return active && 3 * (kxi < 0 ? -kxi : kxi) < N;
+    };
+    cplx<T> U[8], C[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int i = row_of(j);
+        U[j] = C[j] = mk<T>(0, 0);
+        if (kept(i)) {
+            const size_t o = (size_t)ky * N + i;
+            U[j] = __ldcs(u0t + o);
+            if (STAGE > 0) C[j] = __ldcs(acct + o);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) own[j * TT + t] = s ? v[2 * j] : v[2 * j + 1];
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int i = row_of(j);
+        const int kxi = signed_k(i, N);
+        const int akx = kxi < 0 ? -kxi : kxi;
+        const bool keep = active && (3 * akx < N);
+        const T kx = (T)kxi, k2 = kx * kx + kyr * kyr;
+        const cplx<T> mine = s ? v[2 * j + 1] : v[2 * j], other = mate[j * TT + t];
+        cplx<T> nxt = mk<T>(0, 0);
+        if (keep) {
+            const size_t o = (size_t)ky * N + i;
+            const cplx<T> Pm = s ? other : mine, Qm = s ? mine : other;
+            cplx<T> Nl = axpy(kx * kyr, Pm, scl(kx * kx - kyr * kyr, Qm));
+            IFac<T> f = if_factors(tab, nh, akx, ky, -1, k2, p);
+            nxt = lawson_stage<T, STAGE>(p.dt, f, Nl, U[j], C[j]);
+            if (STAGE == 3) __stcs(u0t + o, nxt);
+            else __stcs(acct + o, C[j]);
+        }
+        // psi of the slot: both sequences' next inputs are a wavenumber times it
+        const T ik2 = (keep && k2 > (T)0) ? p.scale / k2 : (T)0;
+        const cplx<T> psi = scl(ik2, nxt);
+        own[N / 2 + j * TT + t] = psi;
+        if (s) v[2 * j + 1] = psi;
+        else v[2 * j] = psi;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const cplx<T> got = mate[N / 2 + j * TT + t];
+        if (s) v[2 * j] = got;
+        else v[2 * j + 1] = got;
+    }
+    // next inputs u = i ky psi (s = 0), v = -i kx psi (s = 1): rounded products, but for slot
+    // 15, whose negated part goes into the first DFT's sums unrounded (of u only with FUSE_U).
+    // That is what the compiler made of one thread per pair (the last slot's products shared a
+    // basic block with the transform); stated here, it keeps every run's bits as they were.
+    T c15 = 0;
+    cplx<T> r15 = mk<T>(0, 0);
+#pragma unroll
+    for (int m = 0; m < 16; ++m) {
+        const T c = s ? -(T)signed_k(k0 + m * TT, N) : kyr;
+        const cplx<T> r = mul_i(v[m]);
+        if (m == 15) {
+            c15 = c;
+            r15 = r;
+        }
+        v[m] = mk<T>(mul_rn(c, r.x), mul_rn(c, r.y));
+    }
+    dft16_fused15(v, c15, r15, FUSE_U && s == 0, s == 1);
+    __syncthreads();  // the traded values are read: the buffers take the exchanges
+    seq_inverse_rest<N>(v, own, t, tw);
+    if (active) {
+#pragma unroll
+        for (int g = 0; g < 16 / RIL; ++g)
+#pragma unroll
+            for (int m = 0; m < RIL; ++m) {
+                const int x = in_pos<N, RIL>(xb, g, m);
+                Xs[2 * xidx(x, ky, kc)] = v[g * RIL + m];
+            }
+    }
+}
+
+// Threads of a column-pass CTA of B columns.
+template <int N, int STAGE, int BX>
+constexpr int col_threads() {
+    return Fused2D<N, BX>::THREADS * (STAGE >= 0 && split_columns<N>() ? 2 : 1);
+}
+
+// Resident CTAs asked for: 768 threads per SM in fp32 with split columns (80 registers; the
+// ensemble above took 3.59 ms with the compiler's own 95, 3.55 with 64).
+template <typename T, int N, int STAGE, int BX>
+constexpr int col_min_blocks() {
+    if (sizeof(T) == 8 || STAGE < 0 || !split_columns<N>()) return 1;
+    const int b = 768 / col_threads<N, STAGE, BX>();
+    return b < 1 ? 1 : b > 16 ? 16 : b;
+}
+
 template <typename T, int N, int STAGE, int BX = 1>
-__global__ void __launch_bounds__(Fused2D<N, BX>::THREADS) k_col_pass(
+__global__ void __launch_bounds__(col_threads<N, STAGE, BX>(), col_min_blocks<T, N, STAGE, BX>()) k_col_pass(
     Pair<T>* __restrict__ X, int kc, cplx<T>* __restrict__ u0t, cplx<T>* __restrict__ acct,
     const T* __restrict__ tab, const StepParams<T>* __restrict__ P,
     const cplx<T>* __restrict__ tw, size_t x_stride, size_t u_stride, int tab_stride) {
     using F = Fused2D<N, BX>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const StepParams<T> p = P[blockIdx.y];
-    col_pass_cols<T, N, STAGE, F::B>(X + blockIdx.y * x_stride, kc, u0t + blockIdx.y * u_stride,
-                                     acct + blockIdx.y * u_stride,
-                                     tab + blockIdx.y * tab_stride, p, tw, blockIdx.x * F::B,
-                                     smem_raw);
+    X += blockIdx.y * x_stride;
+    u0t += blockIdx.y * u_stride;
+    acct += blockIdx.y * u_stride;
+    tab += blockIdx.y * tab_stride;
+    if constexpr (STAGE >= 0 && split_columns<N>())
+        col_pass_split<T, N, STAGE, F::B, (N >= 256 && BX == 1)>(X, kc, u0t, acct, tab, p, tw, blockIdx.x * F::B, smem_raw);
+    else
+        col_pass_cols<T, N, STAGE, F::B>(X, kc, u0t, acct, tab, p, tw, blockIdx.x * F::B, smem_raw);
 }
 
 // ------------------------------------------------------------------------------- streamed column pass

@@ -430,6 +430,25 @@ def test_fused_graph_replays_every_dt_and_amplitude():
     assert s.kernel_launches - launches == 8  # 4 x (row pass + column pass)
 
 
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+@pytest.mark.parametrize("n", [16, 32, 64, 128, 256, 512, 1024])
+def test_split_column_pass_matches_the_general_engine(n, dtype):
+    """The column pass with two threads per pair (n <= 1024): every grid it is compiled for, from
+    one thread per sequence (16) to four warps per column (1024), with forcing, drag and a dt
+    change, against the fp64 cuFFT engine (pinned to the oracle) from the same state."""
+    cfg = Config(n=n, dim=2, nu=1e-3, alpha=0.1, alpha_kmax=2, force_amp=0.2, force_klo=1,
+                 force_khi=3, dtype=dtype)
+    ic = initial.random_phase_2d(n, k0=max(2.0, n / 40), seed=n)
+    out = []
+    for name, c in ((FUSED, cfg), ("b200", cfg.with_(dtype="float64"))):
+        s = get(name).make(c)
+        s.set_state(ic)
+        s.advance(2, 0.2 / n)
+        s.advance(1, 0.1 / n)
+        out.append(s.get_state())
+    assert rel(out[0], out[1]) < TOL[dtype]
+
+
 def test_fused_rejects_what_it_does_not_run():
     for cfg in (Config(n=48, dim=2), Config(n=48, dim=3), Config(n=1024, dim=3),
                 Config(n=8192, dim=2, dtype="float64")):
