@@ -25,9 +25,16 @@ namespace sp {
 
 // Two complex values moved as one unit: aligned to its size so a Pair<float> is one 128-bit
 // access (and a Pair<double> two) instead of separate 64-bit halves.
-template <typename T>
+// PK: its fp32 sums are packed (two fp32 lanes per instruction, the same roundings as two scalar
+// adds, at the scalar lane rate: 121 against 125 lanes per clock and SM): fewer instructions to
+// issue where a pass is bound by issue and latency, at the price of aligned register pairs.
+// Taken where it measured faster: the 3D passes (256^3 rotational, five steps 7.62 -> 7.35 ms;
+// 512^3 Basdevant, two steps 26.5 -> 25.9) and the streamed 2D column pass below n = 8192 (2048^2
+// step 0.179 -> 0.171 ms); single complex sequences and 8192^2 gained nothing.
+template <typename T, bool PK = false>
 struct alignas(4 * sizeof(T) <= 16 ? 4 * sizeof(T) : 16) Pair {
     cplx<T> a, b;
+    __device__ __forceinline__ operator Pair<T, !PK>() const { return Pair<T, !PK>{a, b}; }
 };
 
 // ---------------------------------------------------------------------------- element algebra
@@ -65,22 +72,60 @@ template <int DIR> __device__ __forceinline__ double2 emul_i(double2 x) { return
 __device__ __forceinline__ float2 escale(float2 x, float s) { return scl(s, x); }
 __device__ __forceinline__ double2 escale(double2 x, double s) { return scl(s, x); }
 
-template <typename T>
-__device__ __forceinline__ Pair<T> eadd(Pair<T> x, Pair<T> y) { return {add(x.a, y.a), add(x.b, y.b)}; }
-template <typename T>
-__device__ __forceinline__ Pair<T> esub(Pair<T> x, Pair<T> y) { return {csub(x.a, y.a), csub(x.b, y.b)}; }
-template <typename T>
-__device__ __forceinline__ Pair<T> emul(Pair<T> x, cplx<T> w) { return {cmul(x.a, w), cmul(x.b, w)}; }
+__device__ __forceinline__ float2 add_packed(float2 x, float2 y) {
+    float2 r;
+    asm("{.reg .b64 a, b, c; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; add.rn.f32x2 c, a, b; "
+        "mov.b64 {%0, %1}, c;}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
+    return r;
+}
+__device__ __forceinline__ float2 sub_packed(float2 x, float2 y) {
+    float2 r;
+    asm("{.reg .b64 a, b, c; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; sub.rn.f32x2 c, a, b; "
+        "mov.b64 {%0, %1}, c;}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
+    return r;
+}
+__device__ __forceinline__ double2 add_packed(double2 x, double2 y) { return add(x, y); }
+__device__ __forceinline__ double2 sub_packed(double2 x, double2 y) { return csub(x, y); }
+
+template <typename T, bool K>
+__device__ __forceinline__ Pair<T, K> eadd(Pair<T, K> x, Pair<T, K> y) {
+    if constexpr (K) return {add_packed(x.a, y.a), add_packed(x.b, y.b)};
+    else return {add(x.a, y.a), add(x.b, y.b)};
+}
+template <typename T, bool K>
+__device__ __forceinline__ Pair<T, K> esub(Pair<T, K> x, Pair<T, K> y) {
+    if constexpr (K) return {sub_packed(x.a, y.a), sub_packed(x.b, y.b)};
+    else return {csub(x.a, y.a), csub(x.b, y.b)};
+}
+template <typename T, bool K>
+__device__ __forceinline__ Pair<T, K> emul(Pair<T, K> x, cplx<T> w) { return {cmul(x.a, w), cmul(x.b, w)}; }
+template <int DIR, typename T, bool K>
+__device__ __forceinline__ Pair<T, K> emul_i(Pair<T, K> x) { return {cmul_i<DIR>(x.a), cmul_i<DIR>(x.b)}; }
+template <typename T, bool K>
+__device__ __forceinline__ Pair<T, K> escale(Pair<T, K> x, T s) { return {scl(s, x.a), scl(s, x.b)}; }
+// x + (dir i) y and x - (dir i) y; scalar for every element, so that the swap of y's parts stays
+// a renaming of registers
+template <int DIR, typename E>
+__device__ __forceinline__ E eadd_i(E x, E y) { return eadd(x, emul_i<DIR>(y)); }
+template <int DIR, typename E>
+__device__ __forceinline__ E esub_i(E x, E y) { return esub(x, emul_i<DIR>(y)); }
 template <int DIR, typename T>
-__device__ __forceinline__ Pair<T> emul_i(Pair<T> x) { return {cmul_i<DIR>(x.a), cmul_i<DIR>(x.b)}; }
-template <typename T>
-__device__ __forceinline__ Pair<T> escale(Pair<T> x, T s) { return {scl(s, x.a), scl(s, x.b)}; }
+__device__ __forceinline__ Pair<T, true> eadd_i(Pair<T, true> x, Pair<T, true> y) {
+    return {add(x.a, cmul_i<DIR>(y.a)), add(x.b, cmul_i<DIR>(y.b))};
+}
+template <int DIR, typename T>
+__device__ __forceinline__ Pair<T, true> esub_i(Pair<T, true> x, Pair<T, true> y) {
+    return {csub(x.a, cmul_i<DIR>(y.a)), csub(x.b, cmul_i<DIR>(y.b))};
+}
 
 template <typename E> struct ElemReal;
 template <> struct ElemReal<float2> { using type = float; };
 template <> struct ElemReal<double2> { using type = double; };
-template <> struct ElemReal<Pair<float>> { using type = float; };
-template <> struct ElemReal<Pair<double>> { using type = double; };
+template <typename T, bool K> struct ElemReal<Pair<T, K>> { using type = T; };
 
 // ---------------------------------------------------------------------------- small DFTs
 // X_k = sum_n x_n w^{n k}, w = exp(DIR * 2 pi i / R), in place, natural order in and out.
@@ -93,11 +138,11 @@ __device__ __forceinline__ void dft2(E* x) {
 
 template <int DIR, typename E>
 __device__ __forceinline__ void dft4(E& x0, E& x1, E& x2, E& x3) {
-    E a = eadd(x0, x2), b = esub(x0, x2), c = eadd(x1, x3), d = emul_i<DIR>(esub(x1, x3));
+    E a = eadd(x0, x2), b = esub(x0, x2), c = eadd(x1, x3), d = esub(x1, x3);
     x0 = eadd(a, c);
     x2 = esub(a, c);
-    x1 = eadd(b, d);
-    x3 = esub(b, d);
+    x1 = eadd_i<DIR>(b, d);
+    x3 = esub_i<DIR>(b, d);
 }
 
 template <int DIR, typename E>
@@ -472,8 +517,8 @@ __device__ __forceinline__ void block_fft(E (&v)[16], E* sm, int t, const C* __r
 
 // Exchange between two passes of a Pair transform through a buffer of single complex values
 // (half the bytes of a Pair buffer): the `a` sequences move first, then the `b` sequences.
-template <int N, int R0, int S0, int R1, bool WARP = false, typename T>
-__device__ __forceinline__ void exchange_halves(Pair<T> (&v)[16], cplx<T>* sm, int t) {
+template <int N, int R0, int S0, int R1, bool WARP = false, typename T, bool K>
+__device__ __forceinline__ void exchange_halves(Pair<T, K> (&v)[16], cplx<T>* sm, int t) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         cplx<T> u[16];
@@ -493,8 +538,8 @@ __device__ __forceinline__ void exchange_halves(Pair<T> (&v)[16], cplx<T>* sm, i
 
 // block_fft of Pair elements with the exchanges of exchange_halves: `sm` holds
 // FftPlan<N>::SMEM complex values instead of Pairs.
-template <int N, bool INV, bool WARP = false, bool TWINV = INV, typename T, typename C>
-__device__ __forceinline__ void block_fft_halves(Pair<T> (&v)[16], cplx<T>* sm, int t,
+template <int N, bool INV, bool WARP = false, bool TWINV = INV, typename T, bool K, typename C>
+__device__ __forceinline__ void block_fft_halves(Pair<T, K> (&v)[16], cplx<T>* sm, int t,
                                                  const C* __restrict__ tw) {
     using P = FftPlan<N>;
     static_assert(TWINV == INV || P::R0 == 1, "shared blocks need equal pass structures");
@@ -560,8 +605,8 @@ __device__ __forceinline__ float2 shfl_xor_e(float2 x, int lm) {
 __device__ __forceinline__ double2 shfl_xor_e(double2 x, int lm) {
     return make_double2(shfl_xor_e(x.x, lm), shfl_xor_e(x.y, lm));
 }
-template <typename T>
-__device__ __forceinline__ Pair<T> shfl_xor_e(Pair<T> x, int lm) {
+template <typename T, bool K>
+__device__ __forceinline__ Pair<T, K> shfl_xor_e(Pair<T, K> x, int lm) {
     return {shfl_xor_e(x.a, lm), shfl_xor_e(x.b, lm)};
 }
 

@@ -140,6 +140,11 @@ __device__ __forceinline__ size_t phys_idx(int x, int f, int y, int q) {
 // Z pass: 4 warps (fp32) or 2 (fp64), so its static shared memory stays below 48 KB
 template <typename T>
 constexpr int z_threads() { return sizeof(T) == 4 ? 128 : 64; }
+// and its resident CTAs: five (96 registers) in fp32, four for the Basdevant form at n = 512, which
+// would spill 100 bytes (step at 512^3: rotational 14.0 -> 13.6 ms with five, Basdevant 12.22 ms
+// with four and 12.36 with five; 256^3 Basdevant 1.244 -> 1.208 ms)
+template <typename T, int N, bool ROT>
+constexpr int z_blocks() { return sizeof(T) == 8 ? 1 : (!ROT && N == 512) ? 4 : 5; }
 
 // ------------------------------------------------------------------------------- Y passes
 // A Y pass moves tiles of one field: (x, x+1) x QT adjacent kz pairs x every y, 128 bytes per
@@ -257,7 +262,7 @@ __global__ void __launch_bounds__(YTile<T, N>::THREADS, YTile<T, N>::MIN_BLOCKS)
     tile.template load<ROT, true>(sm, Bs, lt);
     __syncthreads();
     const int kb = spec_base<N>(t), yb = phys_base<N>(t);
-    Pair<T> v[16];
+    Pair<T, true> v[16];
     for_slots([&](auto mc) {
         constexpr int M = decltype(mc)::value;
         auto lo = [&](int k) { return Y::template get<true>(sm, k, u); };
@@ -294,7 +299,7 @@ __global__ void __launch_bounds__(YTile<T, N>::THREADS, YTile<T, N>::MIN_BLOCKS)
     tile.template load<ROT, false>(sm, Bp, lt);
     __syncthreads();
     const int kb = spec_base<N>(t), yb = phys_base<N>(t);
-    Pair<T> v[16];
+    Pair<T, true> v[16];
 #pragma unroll
     for (int g = 0; g < 16 / RF0; ++g)
 #pragma unroll
@@ -372,7 +377,7 @@ __device__ __forceinline__ cplx<T> herm_pair_hi(cplx<T> a, cplx<T> b) {  // a, b
 // MODE 0: the stage's Z pass (inverse, products, forward).  MODE 1: inverse of the velocity
 // only and max |u_i| into umax[0..3) (CFL bound; nothing written back).
 template <typename T, int N, bool ROT, int MODE>
-__global__ void __launch_bounds__(z_threads<T>()) k3_z(Pair<T>* __restrict__ Bp,
+__global__ void __launch_bounds__(z_threads<T>(), z_blocks<T, N, ROT>()) k3_z(Pair<T>* __restrict__ Bp,
                                                        const cplx<T>* __restrict__ tw,
                                                        unsigned long long* __restrict__ umax,
                                                        int want_max) {
@@ -397,7 +402,7 @@ __global__ void __launch_bounds__(z_threads<T>()) k3_z(Pair<T>* __restrict__ Bp,
     const cplx<T> z0 = mk<T>(0, 0);
     const int kb = spec_base<N>(t);  // the z line's samples stay in registers: no sample index
 
-    Pair<T> v[16];
+    Pair<T, true> v[16];
     if constexpr (ROT && MODE == 0) {
         // (omega_y, omega_z) first, kept in shared memory for the products
         cplx<T> w[16];
@@ -637,7 +642,7 @@ __global__ void __launch_bounds__(XPass<T, N, ROT>::THREADS, XPass<T, N, ROT>::M
     if constexpr (STAGE >= 0) {
         if (fw < NFW) {
             const int f = fw;
-            Pair<T> v[16];
+            Pair<T, true> v[16];
 #pragma unroll
             for (int g = 0; g < 16 / RF0; ++g)
 #pragma unroll
@@ -744,7 +749,7 @@ __global__ void __launch_bounds__(XPass<T, N, ROT>::THREADS, XPass<T, N, ROT>::M
     // inverse along x of the next inputs
     if (fw < NIN) {
         const int f = fw;
-        Pair<T> v[16];
+        Pair<T, true> v[16];
         for_slots([&](auto mc) {
             constexpr int M = decltype(mc)::value;
             auto lo = [&](int k) { return st_at(sub, f, k); };
