@@ -253,30 +253,31 @@ __device__ __forceinline__ void stage_weights(unsigned char* sW, const __nv_bflo
     }
 }
 
-// Forward epilogue of a hidden layer: 16 columns c0 .. of row p of Z -> GELU -> bf16 hidden tile.
+// Forward epilogue of a hidden layer: 16 columns c0 .. of row p of Z -> GELU -> bf16 hidden tile;
+// g keeps GELU' for the backward pass.
 __device__ __forceinline__ void epi_forward(uint32_t tbase, uint32_t zcol, unsigned char* sHt,
-                                            int p, int quad, int c0) {
+                                            int p, int quad, int c0, float (&g)[16]) {
     float z[16];
-    tc::tmem_ld16(tc::tmem_at(tbase, 32 * quad, zcol + c0), z);
-    tc::tmem_wait_ld();
-#pragma unroll
-    for (int i = 0; i < 16; ++i) z[i] = gelu(z[i]);
-    st_row8(sHt, p, c0, kK, z);
-    st_row8(sHt, p, c0 + 8, kK, z + 8);
-}
-
-// Backward epilogue: 16 columns of the layer's data gradient times GELU' of its pre-activation.
-__device__ __forceinline__ void epi_backward(uint32_t tbase, uint32_t dcol, uint32_t zcol,
-                                             unsigned char* sDZ, int p, int quad, int c0) {
-    float dh[16], z[16];
-    tc::tmem_ld16(tc::tmem_at(tbase, 32 * quad, dcol + c0), dh);
     tc::tmem_ld16(tc::tmem_at(tbase, 32 * quad, zcol + c0), z);
     tc::tmem_wait_ld();
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
         float h;
-        dh[i] *= gelu_d(z[i], h);
+        g[i] = gelu_d(z[i], h);
+        z[i] = h;
     }
+    st_row8(sHt, p, c0, kK, z);
+    st_row8(sHt, p, c0 + 8, kK, z + 8);
+}
+
+// Backward epilogue: 16 columns of the layer's data gradient times GELU' of its pre-activation.
+__device__ __forceinline__ void epi_backward(uint32_t tbase, uint32_t dcol, unsigned char* sDZ,
+                                             int p, int quad, int c0, const float (&g)[16]) {
+    float dh[16];
+    tc::tmem_ld16(tc::tmem_at(tbase, 32 * quad, dcol + c0), dh);
+    tc::tmem_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) dh[i] *= g[i];
     st_row8(sDZ, p, c0, kH, dh);
     st_row8(sDZ, p, c0 + 8, kH, dh + 8);
 }
@@ -318,8 +319,8 @@ struct TrainSmem {
     static constexpr int X = W + kLayers * kWsz * 2;             // [128 x 80]
     static constexpr int H1 = X + kTile * kK * 2;                // [128 x 80]
     static constexpr int H2 = H1 + kTile * kK * 2;               // [128 x 80]
-    static constexpr int DZ = H2 + kTile * kK * 2;               // [128 x 64]
-    static constexpr int ST = DZ + kTile * kH * 2;               // stencil floats
+    static constexpr int DZ = H2 + kTile * kK * 2;               // 2 x [128 x 64]
+    static constexpr int ST = DZ + 2 * kTile * kH * 2;           // stencil floats
     static constexpr int W4 = ST + kStencil * 4;                 // w4 fp32 [80]
     static constexpr int DW4 = W4 + kK * 4;                      // dw4 partials fp32 [4][80]
     static constexpr int YP = DW4 + 4 * kK * 4;                  // output partials fp32 [4][128]
@@ -338,8 +339,9 @@ constexpr uint32_t kTrainCols = 512;
 // and 16 of the 64 hidden columns each.  The tensor pipe works a few percent of a tile's time;
 // the tile is bound by its GELU epilogues (two MUFU and about twenty fp32 operations for each
 // of some 450 values per point), which four warps, one per scheduler, ran at the latency of
-// their dependency chains.  65536 points: 69.5 -> 55.8 us per
-// launch.
+// their dependency chains.  GELU' of layers 1 and 2 stays in registers from the forward epilogue
+// (32 per thread), so the backward ones evaluate no exponential.  65536 points, launches back to
+// back: 75 us per step with four warps (gradient sum and update included), 58 with sixteen, 52 now.
 constexpr int kTrainThreads = 512;
 constexpr int kTrainGroups = kTrainThreads / kTile;  // column groups of 16
 
@@ -357,7 +359,8 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     unsigned char* sX = smem + TrainSmem::X;
     unsigned char* sH1 = smem + TrainSmem::H1;
     unsigned char* sH2 = smem + TrainSmem::H2;
-    unsigned char* sDZ = smem + TrainSmem::DZ;
+    unsigned char* sDZ = smem + TrainSmem::DZ;                   // dz3, dz1
+    unsigned char* sDZ2 = sDZ + kTile * kH * 2;                  // dz2
     float* sSt = reinterpret_cast<float*>(smem + TrainSmem::ST);
     float* sW4 = reinterpret_cast<float*>(smem + TrainSmem::W4);
     float* sDW4 = reinterpret_cast<float*>(smem + TrainSmem::DW4);
@@ -394,17 +397,19 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     sync_for_mma();
     const uint32_t tb = tslot;
     const uint32_t aX = tc::smem_u32(sX), aH1 = tc::smem_u32(sH1), aH2 = tc::smem_u32(sH2);
-    const uint32_t aDZ = tc::smem_u32(sDZ), aW = tc::smem_u32(sW);
+    const uint32_t aDZ = tc::smem_u32(sDZ), aDZ2 = tc::smem_u32(sDZ2), aW = tc::smem_u32(sW);
     const uint32_t aW1 = aW, aW2 = aW + kWsz * 2, aW3 = aW + 2 * kWsz * 2;
 
     uint32_t phase = 0;
     bool ok = true, first = true;
     float loss = 0.f;
+    float g1[16], g2[16];  // GELU' of layers 1 and 2
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         stencil_store<kTrainThreads>(sSt, nxt, cc);
         const float target = nxt_target * cc.inv_outscale;
         if (tile + (int)gridDim.x < ntiles) load_tile(tile + gridDim.x);
-        __syncthreads();
+        if (first) __syncthreads();
+        else if (!(ok = wait_mma(&bar, phase))) break;  // the last tile's GW1 has read X and dz1
         // ten feature groups of 8 over the four column groups
         if (cg == 0) build_x<0, 3>(sX, sSt, p);
         else if (cg == 1) build_x<3, 6>(sX, sSt, p);
@@ -418,14 +423,14 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
             tc::mma_commit(&bar);
         }
         if (!(ok = wait_mma(&bar, phase))) break;
-        epi_forward(tb, kZ1, sH1, p, quad, c0);
+        epi_forward(tb, kZ1, sH1, p, quad, c0, g1);
         sync_for_mma();
         if (t == 0) {
             issue(tb + kZ2, aH1, 0, kK, aW2, 0, kK, 128, kH, kK / 16, false);
             tc::mma_commit(&bar);
         }
         if (!(ok = wait_mma(&bar, phase))) break;
-        epi_forward(tb, kZ2, sH2, p, quad, c0);
+        epi_forward(tb, kZ2, sH2, p, quad, c0, g2);
         sync_for_mma();
         if (t == 0) {
             issue(tb + kZ3, aH2, 0, kK, aW3, 0, kK, 128, kH, kK / 16, false);
@@ -475,31 +480,33 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
             if (lane == 0) sDW4[quad * kK + kBiasH] += sdy;
         }
 
-        // ---- backward through layers 3, 2, 1
+        // ---- backward through layers 3, 2, 1.  The data gradient goes first and is waited for
+        // alone: the weight gradient's MMAs run beside the next epilogue, which writes the other
+        // dz buffer (a commit also covers every MMA issued before it).
         sync_for_mma();
         if (t == 0) {
-            issue(tb + kGW3, aDZ, 1, kH, aH2, 1, kK, 64, kK, kTile / 16, !first);
             issue(tb + kDH, aDZ, 0, kH, aW3, 1, kK, 128, kK, kH / 16, false);
             tc::mma_commit(&bar);
+            issue(tb + kGW3, aDZ, 1, kH, aH2, 1, kK, 64, kK, kTile / 16, !first);
         }
         if (!(ok = wait_mma(&bar, phase))) break;
-        epi_backward(tb, kDH, kZ2, sDZ, p, quad, c0);
+        epi_backward(tb, kDH, sDZ2, p, quad, c0, g2);
         sync_for_mma();
         if (t == 0) {
-            issue(tb + kGW2, aDZ, 1, kH, aH1, 1, kK, 64, kK, kTile / 16, !first);
-            issue(tb + kDH, aDZ, 0, kH, aW2, 1, kK, 128, kK, kH / 16, false);
+            issue(tb + kDH, aDZ2, 0, kH, aW2, 1, kK, 128, kK, kH / 16, false);
             tc::mma_commit(&bar);
+            issue(tb + kGW2, aDZ2, 1, kH, aH1, 1, kK, 64, kK, kTile / 16, !first);
         }
         if (!(ok = wait_mma(&bar, phase))) break;
-        epi_backward(tb, kDH, kZ1, sDZ, p, quad, c0);
+        epi_backward(tb, kDH, sDZ, p, quad, c0, g1);
         sync_for_mma();
         if (t == 0) {
             issue(tb + kGW1, aDZ, 1, kH, aX, 1, kK, 64, kK, kTile / 16, !first);
-            tc::mma_commit(&bar);
+            tc::mma_commit(&bar);  // waited for at the next tile's X, or after the last tile
         }
-        if (!(ok = wait_mma(&bar, phase))) break;
         first = false;
     }
+    if (ok && !first) ok = wait_mma(&bar, phase);
 
     if (ok) {
         float* out = partials + (size_t)blockIdx.x * kPartStride;
