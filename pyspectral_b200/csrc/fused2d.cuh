@@ -180,6 +180,7 @@ __device__ __forceinline__ void row_pass_rows(Pair<T>* __restrict__ X, int row0,
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
             const int c = m * TT;
+            if (c >= KC && c + TT - 1 <= N - KC) continue;  // dealiased: not read below
             if (c % 16 == 0) st[c + (c >> 4)] = v[m];
             else sm[spad(k0 + c)] = v[m];
         }
