@@ -171,8 +171,10 @@ struct YTile {
     static constexpr int CPP = (int)sizeof(Pair<T>) / 16;        // chunks per Pair
     static constexpr size_t BYTES = (size_t)N * 128;
     static constexpr size_t SMEM = KT * BYTES;
-    // shared memory holds three CTAs of 64 KB per SM (n = 512 fp32, n >= 256 fp64), 32 KB else
-    static constexpr int MIN_BLOCKS = sizeof(T) == 4 ? (THREADS > 128 ? 3 : 5) : 2;
+    // shared memory holds three CTAs of 64 KB per SM (n = 512 fp32, all fp64), more of 32 KB; fp64
+    // at 168 registers (step: 256^3 Basdevant 2.58 -> 2.48 ms, 128^3 rotational 0.424 -> 0.416
+    // against the compiler's own 230)
+    static constexpr int MIN_BLOCKS = sizeof(T) == 4 && THREADS == 128 ? 5 : 3;
     static_assert(FftPlan<N>::SMEM * sizeof(cplx<T>) <= BYTES / UN, "exchange fits the tile");
     int x2, f, q0;
     bool active;
