@@ -28,9 +28,9 @@ namespace sp {
 // PK: its fp32 sums are packed (two fp32 lanes per instruction, the same roundings as two scalar
 // adds, at the scalar lane rate: 121 against 125 lanes per clock and SM): fewer instructions to
 // issue where a pass is bound by issue and latency, at the price of aligned register pairs.
-// Taken where it measured faster: the 3D passes (256^3 rotational, five steps 7.62 -> 7.35 ms;
-// 512^3 Basdevant, two steps 26.5 -> 25.9) and the streamed 2D column pass below n = 8192 (2048^2
-// step 0.179 -> 0.171 ms); single complex sequences and 8192^2 gained nothing.
+// Taken in the 3D Y and X passes (256^3: k3_yfwd 45 -> 40 us, k3_yinv 74 -> 71; 512^3: k3_yfwd 613
+// -> 566 us, k3_x 6 %), whose sums take no product, so that packing changes no rounding; elsewhere
+// the compiler fuses products into scalar sums, and results would move.
 template <typename T, bool PK = false>
 struct alignas(4 * sizeof(T) <= 16 ? 4 * sizeof(T) : 16) Pair {
     cplx<T> a, b;

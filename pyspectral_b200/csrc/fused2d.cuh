@@ -311,8 +311,8 @@ __device__ __forceinline__ Pair<T> next_inputs(T kx, T ky, T k2, bool keep, cplx
 // inverse-transform inputs written back into v.
 // ld_u(i, o) / ld_c(i, o): the state / accumulator value of kept row i (o = its global index);
 // the updated values go to global memory.
-template <typename T, int N, int STAGE, bool K, typename LdU, typename LdC>
-__device__ __forceinline__ void col_update_from(Pair<T, K> (&v)[16], int k0, int ky, bool active,
+template <typename T, int N, int STAGE, typename LdU, typename LdC>
+__device__ __forceinline__ void col_update_from(Pair<T> (&v)[16], int k0, int ky, bool active,
                                                 cplx<T>* __restrict__ u0t,
                                                 cplx<T>* __restrict__ acct,
                                                 const T* __restrict__ tab,
@@ -623,8 +623,6 @@ k_col_stream(const __grid_constant__ CUtensorMap xmap, Pair<T>* __restrict__ X, 
              unsigned* __restrict__ err) {
     static_assert(STAGE >= 0, "the set-up pass reads no X");
     using CS = ColStream<T, N>;
-    // packed sums where the registers allow (at n = 8192 they spill)
-    constexpr bool PACK = N < 8192;
     constexpr int RF0 = first_radix<N, false>();
     constexpr int RIL = last_radix<N, true>();
     constexpr int BW = stream_box_w<T>(), BH = stream_box_h<N>();
@@ -698,7 +696,7 @@ k_col_stream(const __grid_constant__ CUtensorMap xmap, Pair<T>* __restrict__ X, 
             return;
         }
         px ^= 1u;
-        Pair<T, PACK> v[16];
+        Pair<T> v[16];
 #pragma unroll
         for (int g = 0; g < 16 / RF0; ++g)
 #pragma unroll

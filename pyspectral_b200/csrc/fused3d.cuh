@@ -56,8 +56,7 @@ struct Dims {
 };
 
 // Field slots of the work arrays: Basdevant 5 (u, v, w in; 5 stress components out),
-// rotational 6 (u, omega in; u x omega out).  Slots (0, 1), Basdevant outputs (2, 3) and
-// rotational inputs (4, 5) hold the combinations of a pair of fields (see k3_z).
+// rotational 6 (u, omega in; u x omega out).
 template <bool ROT> constexpr int nslot() { return ROT ? 6 : 5; }
 template <bool ROT> constexpr int ninv() { return ROT ? 6 : 3; }
 template <bool ROT> constexpr int nfwd() { return ROT ? 3 : 5; }
@@ -140,11 +139,6 @@ __device__ __forceinline__ size_t phys_idx(int x, int f, int y, int q) {
 // Z pass: 4 warps (fp32) or 2 (fp64), so its static shared memory stays below 48 KB
 template <typename T>
 constexpr int z_threads() { return sizeof(T) == 4 ? 128 : 64; }
-// and its resident CTAs: five (96 registers) in fp32, four for the Basdevant form at n = 512, which
-// would spill 100 bytes (step at 512^3: rotational 14.0 -> 13.6 ms with five, Basdevant 12.22 ms
-// with four and 12.36 with five; 256^3 Basdevant 1.244 -> 1.208 ms)
-template <typename T, int N, bool ROT>
-constexpr int z_blocks() { return sizeof(T) == 8 ? 1 : (!ROT && N == 512) ? 4 : 5; }
 
 // ------------------------------------------------------------------------------- Y passes
 // A Y pass moves tiles of one field: (x, x+1) x QT adjacent kz pairs x every y, 128 bytes per
@@ -325,47 +319,8 @@ __device__ __forceinline__ unsigned long long max_bits(double m, bool nan) {
     return nan ? 0x7ff8000000000000ull : (unsigned long long)__double_as_longlong(m);
 }
 
-// Pairs of real fields (f, g) whose transform along z is one complex transform of f + i g are
-// kept in the work arrays as the combinations a = F + i G and b = F - i G of their half spectra
-// (kz <= KM): the value of Z = F[f + i g] at FFT index k is a(k) for k <= KM and conj b(n - k)
-// for k >= n - KM, so the Z pass moves each value once, with no Hermitian completion of its
-// input and no splitting of its output.  The combinations are linear: they pass through the y
-// and x transforms, and the X pass forms F and G in registers.  Only fields of the same kind
-// are paired (velocities, vorticities, stresses), as the transform along z pairs them.
-// The pass is bound by instruction issue: with the half spectra stored instead (two reads and
-// four adds per completed value, two exchanges through shared memory to split the outputs)
-// 512^3 fp32 Basdevant took 1.29 ms, now 1.09; 256^3 rotational 0.121 -> 0.114 ms.
-template <typename C>
-__device__ __forceinline__ C conj(C z) {
-    z.y = -z.y;
-    return z;
-}
-// Z(0) = Re F(0) + i Re G(0): c2r ignores the imaginary parts at k = 0
-template <typename C>
-__device__ __forceinline__ C pair_mean(C a, C b) {
-    using R = decltype(a.x);
-    C r;
-    r.x = (R)0.5 * (a.x + b.x);
-    r.y = (R)0.5 * (a.y - b.y);
-    return r;
-}
-template <typename C>
-__device__ __forceinline__ void combine(C f, C g, C& a, C& b) {
-    a.x = f.x - g.y;
-    a.y = f.y + g.x;
-    b.x = f.x + g.y;
-    b.y = f.y - g.x;
-}
-template <typename C>
-__device__ __forceinline__ void uncombine(C a, C b, C& f, C& g) {
-    using R = decltype(a.x);
-    f.x = (R)0.5 * (a.x + b.x);
-    f.y = (R)0.5 * (a.y + b.y);
-    g.x = (R)0.5 * (a.y - b.y);
-    g.y = (R)0.5 * (b.x - a.x);
-}
-// Hermitian completion along z of two real fields kept as half spectra a(kz), b(kz) (kz <= KM):
-// the value at FFT index k of A + i B.
+// Hermitian completion along z of two real fields' half spectra a(kz), b(kz) (kz <= KM): the
+// value at FFT index k of Z = A + i B.
 template <typename T>
 __device__ __forceinline__ cplx<T> herm_pair_lo(cplx<T> a, cplx<T> b, int k) {
     if (k == 0) return mk<T>(a.x, b.x);  // c2r ignores Im at k = 0
@@ -379,7 +334,7 @@ __device__ __forceinline__ cplx<T> herm_pair_hi(cplx<T> a, cplx<T> b) {  // a, b
 // MODE 0: the stage's Z pass (inverse, products, forward).  MODE 1: inverse of the velocity
 // only and max |u_i| into umax[0..3) (CFL bound; nothing written back).
 template <typename T, int N, bool ROT, int MODE>
-__global__ void __launch_bounds__(z_threads<T>(), z_blocks<T, N, ROT>()) k3_z(Pair<T>* __restrict__ Bp,
+__global__ void __launch_bounds__(z_threads<T>()) k3_z(Pair<T>* __restrict__ Bp,
                                                        const cplx<T>* __restrict__ tw,
                                                        unsigned long long* __restrict__ umax,
                                                        int want_max) {
@@ -404,16 +359,14 @@ __global__ void __launch_bounds__(z_threads<T>(), z_blocks<T, N, ROT>()) k3_z(Pa
     const cplx<T> z0 = mk<T>(0, 0);
     const int kb = spec_base<N>(t);  // the z line's samples stay in registers: no sample index
 
-    Pair<T, true> v[16];
+    Pair<T> v[16];
     if constexpr (ROT && MODE == 0) {
         // (omega_y, omega_z) first, kept in shared memory for the products
         cplx<T> w[16];
         for_slots([&](auto mc) {
             constexpr int M = decltype(mc)::value;
-            auto lo = [&](int k) {
-                return M == 0 && k == 0 ? pair_mean(B[at(4, 0)], B[at(5, 0)]) : B[at(4, k)];
-            };
-            auto hi = [&](int k) { return conj(B[at(5, N - k)]); };
+            auto lo = [&](int k) { return herm_pair_lo<T>(B[at(4, k)], B[at(5, k)], k); };
+            auto hi = [&](int k) { return herm_pair_hi<T>(B[at(4, N - k)], B[at(5, N - k)]); };
             w[M] = active ? slot_value<N, M>(kb, lo, hi, z0) : z0;
         });
         seq_fft<N, true, true>(w, sm, t, tw);
@@ -424,9 +377,9 @@ __global__ void __launch_bounds__(z_threads<T>(), z_blocks<T, N, ROT>()) k3_z(Pa
         constexpr int M = decltype(mc)::value;
         auto lo = [&](int k) {
             cplx<T> wz;
-            if (ROT && MODE == 0) wz = herm_pair_lo<T>(B[at(2, k)], B[at(3, k)], M == 0 ? k : 1);
-            else wz = M == 0 && k == 0 ? mk<T>(B[at(2, 0)].x, (T)0) : B[at(2, k)];
-            return Pair<T>{M == 0 && k == 0 ? pair_mean(B[at(0, 0)], B[at(1, 0)]) : B[at(0, k)], wz};
+            if (ROT && MODE == 0) wz = herm_pair_lo<T>(B[at(2, k)], B[at(3, k)], k);
+            else wz = k == 0 ? mk<T>(B[at(2, 0)].x, (T)0) : B[at(2, k)];
+            return Pair<T>{herm_pair_lo<T>(B[at(0, k)], B[at(1, k)], k), wz};
         };
         auto hi = [&](int k) {
             const int kk = N - k;
@@ -437,7 +390,7 @@ __global__ void __launch_bounds__(z_threads<T>(), z_blocks<T, N, ROT>()) k3_z(Pa
                 const cplx<T> c = B[at(2, kk)];
                 wz = mk<T>(c.x, -c.y);
             }
-            return Pair<T>{conj(B[at(1, kk)]), wz};
+            return Pair<T>{herm_pair_hi<T>(B[at(0, kk)], B[at(1, kk)]), wz};
         };
         v[M] = active ? slot_value<N, M>(kb, lo, hi, pzero<T>()) : pzero<T>();
     });
@@ -492,20 +445,24 @@ __global__ void __launch_bounds__(z_threads<T>(), z_blocks<T, N, ROT>()) k3_z(Pa
             }
         }
         seq_fft<N, false, true>(v, sm, t, tw);  // output slot M: k = kb + M n/16
-        // Z' = F[p + i q] to its combinations: a(k) = Z'(k), b(k) = conj Z'(n - k), k < KZ
-        if (active) {
-            for_slots([&](auto mc) {
-                constexpr int M = decltype(mc)::value;
-                constexpr int LO = M * TT, HI = LO + TT - 1;
-                const int k = kb + LO;
-                auto put = [&](int f, cplx<T> z) {
-                    if (LO < D::KZ && k < D::KZ) B[at(f, k)] = z;
-                    if (M == 0 && k == 0) B[at(f + 1, 0)] = conj(z);
-                    if (HI > N - D::KZ && k > N - D::KZ) B[at(f + 1, N - k)] = conj(z);
-                };
-                put(0, v[M].a);
-                if (!ROT) put(2, v[M].b);
-            });
+        // split Z' = F(p + i q): P(k) = (Z'(k) + conj Z'(n-k)) / 2,
+        // Q(k) = (Z'(k) - conj Z'(n-k)) / 2i
+        constexpr int NSPLIT = ROT ? 1 : 2;
+#pragma unroll
+        for (int h = 0; h < NSPLIT; ++h) {
+            __syncwarp();
+#pragma unroll
+            for (int e = 0; e < 16; ++e) sm[spad(kb + e * TT)] = h == 0 ? v[e].a : v[e].b;
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < (D::KZ + TT - 1) / TT; ++j) {
+                const int k = t + j * TT;
+                if (active && ((j + 1) * TT <= D::KZ || k < D::KZ)) {
+                    const cplx<T> a = sm[spad(k)], b = sm[spad((N - k) & (N - 1))];
+                    B[at(2 * h, k)] = mk<T>((T)0.5 * (a.x + b.x), (T)0.5 * (a.y - b.y));
+                    B[at(2 * h + 1, k)] = mk<T>((T)0.5 * (a.y + b.y), (T)0.5 * (b.x - a.x));
+                }
+            }
         }
         if constexpr (ROT) {
             // the third product had a zero imaginary part: its r2c coefficients are Z'(k)
@@ -690,13 +647,11 @@ __global__ void __launch_bounds__(XPass<T, N, ROT>::THREADS, XPass<T, N, ROT>::M
                 }
                 cplx<T> N0, N1, N2;
                 if constexpr (ROT) {
-                    uncombine(F[0], F[1], N0, N1);
+                    N0 = F[0];
+                    N1 = F[1];
                     N2 = F[2];
                 } else {
-                    cplx<T> t11, t22, t12, t13;
-                    const cplx<T> t23 = F[4];
-                    uncombine(F[0], F[1], t11, t22);
-                    uncombine(F[2], F[3], t12, t13);
+                    const cplx<T> t11 = F[0], t22 = F[1], t12 = F[2], t13 = F[3], t23 = F[4];
                     const cplx<T> t33 = mk<T>(-(t11.x + t22.x), -(t11.y + t22.y));
                     N0 = mul_mi(add(add(scl(kx, t11), scl(ky, t12)), scl(kz, t13)));
                     N1 = mul_mi(add(add(scl(kx, t12), scl(ky, t22)), scl(kz, t23)));
@@ -725,18 +680,18 @@ __global__ void __launch_bounds__(XPass<T, N, ROT>::THREADS, XPass<T, N, ROT>::M
                     acc[2 * CS + o] = Cc;
                 }
             }
-            // next inputs: u scaled (u, v as combinations); rotational form also omega = i k x u
-            // (omega_y, omega_z as combinations)
+            // next inputs: u scaled; rotational form also omega = i k x u
             const T sc = p.scale;
             a = scl(sc, a);
             b = scl(sc, b);
             c = scl(sc, c);
-            combine(a, b, out[0], out[1]);
+            out[0] = a;
+            out[1] = b;
             out[2] = c;
             if (ROT) {
                 out[3] = mul_i(add(scl(ky, c), scl(-kz, b)));
-                const cplx<T> oy = mul_i(add(scl(kz, a), scl(-kx, c)));
-                combine(oy, mul_i(add(scl(kx, b), scl(-ky, a))), out[4], out[5]);
+                out[4] = mul_i(add(scl(kz, a), scl(-kx, c)));
+                out[5] = mul_i(add(scl(kx, b), scl(-ky, a)));
             }
         }
 #pragma unroll
