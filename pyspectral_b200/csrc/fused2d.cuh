@@ -416,9 +416,11 @@ __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(
 // Grids whose column pass gives each of a column's two sequences its own threads.  Above, the
 // streamed pass's prefetch buffer leaves no room for two exchange buffers, and it is faster than
 // this pass without the prefetch (2048^2 fp32 0.173 against 0.187 ms per step, 4096^2 0.651
-// against 0.833).
+// against 0.833).  n = 16 keeps one thread per pair: its wavenumbers are constants of the unrolled
+// slots, and the sums there take other unrounded products than those stated below (20.8 us per
+// step, 16.7 with two threads, but other last bits).
 template <int N>
-constexpr bool split_columns() { return N <= 1024; }
+constexpr bool split_columns() { return N >= 32 && N <= 1024; }
 
 // The column pass (stages 0..3) with 2 (n/16) threads per column: thread s n/16 + t transforms
 // sequence s of the pair (P, Q) forward and of (u, v) back, and updates the slots m = s (mod 2) of
