@@ -432,7 +432,7 @@ constexpr bool split_columns() { return N >= 32 && N <= 1024; }
 // large ones by the warps that registers leave resident.  One B200, per step: 64^2 fp64 45.5 -> 31
 // us, 256^2 fp64 49 -> 37 us, 512^2 fp32 54.7 -> 43.6 us; ensemble of 64 runs each at 128^2..1024^2
 // fp32 3.78 -> 3.53 ms.
-template <typename T, int N, int STAGE, int B, bool FUSE_U>
+template <typename T, int N, int STAGE, int B>
 __device__ __forceinline__ void col_pass_split(Pair<T>* __restrict__ X, int kc,
                                                cplx<T>* __restrict__ u0t,
                                                cplx<T>* __restrict__ acct,
@@ -519,9 +519,10 @@ __device__ __forceinline__ void col_pass_split(Pair<T>* __restrict__ X, int kc,
         else v[2 * j + 1] = got;
     }
     // next inputs u = i ky psi (s = 0), v = -i kx psi (s = 1): rounded products, but for slot
-    // 15, whose negated part goes into the first DFT's sums unrounded (of u only with FUSE_U).
-    // That is what the compiler made of one thread per pair (the last slot's products shared a
-    // basic block with the transform); stated here, it keeps every run's bits as they were.
+    // 15, whose product goes into the first DFT's sums unrounded (u's only where a CTA holds one
+    // column, B = 1, and ky is uniform over the CTA).  These are the roundings of the pass with one
+    // thread per pair as compiled, found by comparing states over n, tiles and precisions: a
+    // run's bits do not change from version to version (tests/golden/state_bits.json pins them).
     T c15 = 0;
     cplx<T> r15 = mk<T>(0, 0);
 #pragma unroll
@@ -534,7 +535,7 @@ __device__ __forceinline__ void col_pass_split(Pair<T>* __restrict__ X, int kc,
         }
         v[m] = mk<T>(mul_rn(c, r.x), mul_rn(c, r.y));
     }
-    dft16_fused15(v, c15, r15, FUSE_U && s == 0, s == 1);
+    dft16_fused15(v, c15, r15, B == 1 && s == 0, s == 1);
     __syncthreads();  // the traded values are read: the buffers take the exchanges
     seq_inverse_rest<N>(v, own, t, tw);
     if (active) {
@@ -576,7 +577,7 @@ __global__ void __launch_bounds__(col_threads<N, STAGE, BX>(), col_min_blocks<T,
     acct += blockIdx.y * u_stride;
     tab += blockIdx.y * tab_stride;
     if constexpr (STAGE >= 0 && split_columns<N>())
-        col_pass_split<T, N, STAGE, F::B, (N >= 256 && BX == 1)>(X, kc, u0t, acct, tab, p, tw, blockIdx.x * F::B, smem_raw);
+        col_pass_split<T, N, STAGE, F::B>(X, kc, u0t, acct, tab, p, tw, blockIdx.x * F::B, smem_raw);
     else
         col_pass_cols<T, N, STAGE, F::B>(X, kc, u0t, acct, tab, p, tw, blockIdx.x * F::B, smem_raw);
 }
