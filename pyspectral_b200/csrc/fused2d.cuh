@@ -555,11 +555,15 @@ constexpr int col_threads() {
     return Fused2D<N, BX>::THREADS * (STAGE >= 0 && split_columns<N>() ? 2 : 1);
 }
 
-// Resident CTAs asked for: 768 threads per SM in fp32 with split columns (80 registers; the
-// ensemble above took 3.59 ms with the compiler's own 95, 3.55 with 64).
+// Resident CTAs asked for.  fp32 with split columns: 768 threads per SM at 80 registers (the
+// ensemble above took 3.59 ms with the compiler's own 95, 3.55 with 64), but no more than 16 CTAs,
+// 512 threads at 120 registers where a CTA is one warp (n = 256), and one CTA of 512 (n = 1024,
+// tile 4).  One thread per pair: the compiler's own registers, 0; asking for one CTA gave 4096^2
+// fp32 143-152 of them for 103-106, and one resident CTA for two.
 template <typename T, int N, int STAGE, int BX>
 constexpr int col_min_blocks() {
-    if (sizeof(T) == 8 || STAGE < 0 || !split_columns<N>()) return 1;
+    if (STAGE < 0 || !split_columns<N>()) return 0;
+    if (sizeof(T) == 8) return 1;
     const int b = 768 / col_threads<N, STAGE, BX>();
     return b < 1 ? 1 : b > 16 ? 16 : b;
 }
