@@ -159,7 +159,10 @@ struct YTile {
     static constexpr int QT = sizeof(T) == 4 ? 4 : 2;            // kz pairs
     static constexpr int UN = 2 * QT;                            // transforms
     static constexpr int PT = UN * D::T;                         // threads
-    static constexpr int KT = PT >= 128 ? 1 : 128 / PT;          // tiles per CTA
+    // one warp per CTA at n <= 64, where CTAs of 128 threads leave SMs empty: fp32 Basdevant step
+    // 69.7 -> 65.6 us at 16^3, 71.7 -> 69.2 at 32^3 (the direct passes before the tiles: 69.7, 73.8)
+    static constexpr int CTA = N <= 64 ? 32 : 128;
+    static constexpr int KT = PT >= CTA ? 1 : CTA / PT;          // tiles per CTA
     static constexpr int THREADS = PT * KT;
     static constexpr int NB = (D::NQ + QT - 1) / QT;             // tiles per (x pair, field)
     static constexpr int CPP = (int)sizeof(Pair<T>) / 16;        // chunks per Pair
@@ -168,7 +171,7 @@ struct YTile {
     // shared memory holds three CTAs of 64 KB per SM (n = 512 fp32, all fp64), more of 32 KB; fp64
     // at 168 registers (step: 256^3 Basdevant 2.58 -> 2.48 ms, 128^3 rotational 0.424 -> 0.416
     // against the compiler's own 230)
-    static constexpr int MIN_BLOCKS = sizeof(T) == 4 && THREADS == 128 ? 5 : 3;
+    static constexpr int MIN_BLOCKS = THREADS > 128 ? 3 : (sizeof(T) == 4 ? 640 : 384) / THREADS;
     static_assert(FftPlan<N>::SMEM * sizeof(cplx<T>) <= BYTES / UN, "exchange fits the tile");
     int x2, f, q0;
     bool active;
