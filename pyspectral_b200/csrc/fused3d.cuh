@@ -515,11 +515,16 @@ struct XPass {
     static constexpr int U = G * S;
     static constexpr int WARPS = G * nslot<ROT>();
     static constexpr int THREADS = WARPS * 32;
-    // fp32: as many CTAs as leave a thread about 100 registers; fp64: two
-    static constexpr int MIN_BLOCKS = sizeof(T) == 8 ? 2 : 20 / WARPS;
     static constexpr int ROW = D::KK;  // Pairs
     static constexpr size_t smem_bytes() { return (size_t)U * nslot<ROT>() * ROW * sizeof(Pair<T>); }
     static constexpr int UNITS = D::KK * D::NQ;
+    // fp64: two CTAs.  fp32: as many as 20 warps hold, 96 registers a thread, spilling up to 90
+    // bytes of it: at stage 1 against two CTAs without a spill, 128^3 Basdevant 19.0 and 21.2 us,
+    // 256^3 94 and 119, 256^3 rotational 119.3 and 120.2; three CTAs or the compiler's own
+    // registers (141-148, 96-114 at 512^3) 101 and more, 1.09 and 1.15-1.26 ms at 512^3 Basdevant.
+    // A grid that one CTA per SM holds (n <= 64) gains nothing from the warps: two CTAs there
+    // (64^3 Basdevant 9.9 -> 8.7 us, rotational 9.3 -> 8.8).
+    static constexpr int MIN_BLOCKS = sizeof(T) == 8 || (UNITS + U - 1) / U <= 148 ? 2 : 20 / WARPS;
     static_assert(FftPlan<N>::SMEM * sizeof(cplx<T>) <= ROW * sizeof(Pair<T>), "exchange fits a row");
 };
 
