@@ -87,6 +87,9 @@ enum sp_diag_index {
 
 /* ABI version of the loaded library (SP_ABI_VERSION at build time). */
 int sp_abi_version(void);
+/* Short hash of the sources and compiler flags the library was built from ("" when the build did
+ * not define SP_SOURCE_REVISION): measurements of its kernels are kept under it. */
+const char* sp_source_revision(void);
 
 /* Create an engine for one grid.  Replaces CupyCudaSolver.__init__'s plan and kernel set-up
  * (src/pyspectral/backends/cupy_cuda.py:40-82, plans :100-112).  Requires a CUDA device;

@@ -32,6 +32,7 @@ _dp = ctypes.POINTER(ctypes.c_double)
 # name -> (restype, argtypes); the exported C ABI
 SIGNATURES: dict[str, tuple[Any, list[Any]]] = {
     "sp_abi_version": (_i, []),
+    "sp_source_revision": (ctypes.c_char_p, []),
     "sp_create": (_vp, [_i, _i, _i, _i, _i, ctypes.POINTER(_i)]),
     "sp_destroy": (None, [_vp]),
     "sp_query_sizes": (_i, [_vp, ctypes.POINTER(ctypes.c_int64), _i]),

@@ -7,6 +7,7 @@ always rebuilds).  nvcc cross-compiles, so this runs on a machine without a GPU.
 
 from __future__ import annotations
 
+import hashlib
 import os
 import shutil
 import subprocess
@@ -47,9 +48,22 @@ def needs_build(lib: Path = LIB) -> bool:
     return any(p.stat().st_mtime > t for p in _deps())
 
 
+CODEGEN = [*ARCH, "-lineinfo", "-O3", "-std=c++20", "--expt-relaxed-constexpr",
+           "-Xcompiler", "-fPIC,-O3,-Wall"]
+
+
+def source_revision() -> str:
+    """Short hash of every source and header and of the compiler flags: the revision a library
+    built now reports (``sp_source_revision``)."""
+    h = hashlib.sha256(" ".join(CODEGEN).encode())
+    for p in _deps():
+        h.update(p.name.encode() + b"\0" + p.read_bytes() + b"\0")
+    return "r" + h.hexdigest()[:12]
+
+
 def _flags(extra: list[str] | None = None) -> list[str]:
-    return [*ARCH, "-lineinfo", "-O3", "-std=c++20", "--expt-relaxed-constexpr",
-            "-Xcompiler", "-fPIC,-O3,-Wall", f"-I{INCLUDE}", f"-I{CSRC}", *(extra or [])]
+    return [*CODEGEN, f"-DSP_SOURCE_REVISION={source_revision()}", f"-I{INCLUDE}", f"-I{CSRC}",
+            *(extra or [])]
 
 
 def command(out: Path = LIB, extra: list[str] | None = None) -> list[str]:

@@ -704,6 +704,13 @@ extern "C" {
 
 int sp_abi_version(void) { return SP_ABI_VERSION; }
 
+#ifndef SP_SOURCE_REVISION
+#define SP_SOURCE_REVISION
+#endif
+#define SP_TEXT(x) #x
+#define SP_TEXT_OF(x) SP_TEXT(x)
+const char* sp_source_revision(void) { return SP_TEXT_OF(SP_SOURCE_REVISION); }
+
 const char* sp_create_error(void) { return g_create_error.c_str(); }
 
 const char* sp_last_error(const sp_solver* s) { return s ? s->err.c_str() : "null handle"; }

@@ -78,7 +78,9 @@ class TileTuner:
     """Chooses each size class's tile (sub-blocks per CTA of the fused row and column passes,
     1, 2 or 4 times the default) by timing the class's batched step on the device (CUDA
     events, ``reps`` steps after two warm-up steps); choices are cached in a JSON file keyed by
-    GPU model, grid, precision and member count.  Tiles change results at round-off only."""
+    GPU model, grid, precision and member count, each with the revision of the library whose
+    kernels were timed: an entry of another revision is timed again.  Tiles change results at
+    round-off only."""
 
     def __init__(self, path: Path | None = None, reps: int = 5) -> None:
         self.path = Path(path) if path is not None else tune_cache_path()
@@ -86,15 +88,24 @@ class TileTuner:
         self.cache = load_tune_cache(self.path)
         self.report: dict[str, Any] = {}
 
+    def _cached(self, key: str, what: str, cands: list[int], revision: str) -> int | None:
+        """The cached choice, if it was timed with this library's kernels."""
+        hit = self.cache.get(key)
+        if not isinstance(hit, dict) or hit.get("revision") != revision or \
+                hit.get(what) not in cands:
+            return None
+        self.report[key] = dict(hit, cached=True)
+        return int(hit[what])
+
     def choose(self, sc: _SizeClass, stream: Any) -> int:
         torch, lib = sc.torch, sc.lib
         gpu = torch.cuda.get_device_name(sc.u0.device)
         key = tune_key(gpu, sc.n, sc.fp64, sc.count)
         cands = [t for t in TILES if lib.sp_batch_tile_supported(sc.n, t)]
-        hit = self.cache.get(key)
-        if isinstance(hit, dict) and hit.get("tile") in cands:
-            self.report[key] = dict(hit, cached=True)
-            return int(hit["tile"])
+        rev = (lib.sp_source_revision() or b"").decode()
+        hit = self._cached(key, "tile", cands, rev)
+        if hit is not None:
+            return hit
         if len(cands) == 1:
             return cands[0]
         sc.set_step(np.full(sc.count, 1e-4), np.zeros(sc.count), stream)
@@ -113,7 +124,7 @@ class TileTuner:
             e1.synchronize()
             times[t] = e0.elapsed_time(e1) / self.reps
         best = min(times, key=times.get)
-        entry = {"tile": best, "ms_per_step": {str(k): v for k, v in times.items()}}
+        entry = {"tile": best, "revision": rev, "ms_per_step": {str(k): v for k, v in times.items()}}
         self.cache[key] = entry
         self.report[key] = dict(entry, cached=False)
         save_tune_cache(self.path, self.cache)
@@ -123,16 +134,17 @@ class TileTuner:
     def choose_worklist(self, ens: Ensemble) -> int:
         """The group step's form: the work-list passes with CTAs of 64 or 128 threads, or one
         launch per class and phase (0) — whichever steps the group fastest (CUDA events,
-        ``reps`` group steps after two warm-up steps); cached per GPU model and class set."""
+        ``reps`` group steps after two warm-up steps); cached per GPU model, class set and
+        library revision."""
         torch, lib = ens.torch, ens.lib
         gpu = torch.cuda.get_device_name(ens.device)
         sig = ",".join(f"{c.n}{'d' if c.fp64 else 'f'}x{c.count}" for c in ens.classes)
         key = f"{gpu}|group|{sig}"
         cands = [0] + [mt for mt in (64, 128) if ens._worklist_ok(mt)]
-        hit = self.cache.get(key)
-        if isinstance(hit, dict) and hit.get("worklist") in cands:
-            self.report[key] = dict(hit, cached=True)
-            return int(hit["worklist"])
+        rev = (lib.sp_source_revision() or b"").decode()
+        hit = self._cached(key, "worklist", cands, rev)
+        if hit is not None:
+            return hit
         if len(cands) == 1:
             return 0
         st = ens._stream()
@@ -153,7 +165,7 @@ class TileTuner:
             e1.synchronize()
             times[mt] = e0.elapsed_time(e1) / self.reps
         best = min(times, key=times.get)
-        entry = {"worklist": best, "ms_per_step": {str(k): v for k, v in times.items()}}
+        entry = {"worklist": best, "revision": rev, "ms_per_step": {str(k): v for k, v in times.items()}}
         self.cache[key] = entry
         self.report[key] = dict(entry, cached=False)
         save_tune_cache(self.path, self.cache)

@@ -48,6 +48,11 @@ def test_abi_version(lib):
     assert lib.sp_abi_version() == 1
 
 
+def test_source_revision(lib):
+    """The library names the sources and flags it was built from (a key of kept timings)."""
+    assert re.fullmatch(rb"r[0-9a-f]{12}", lib.sp_source_revision())
+
+
 def test_library_targets_sm100a_only():
     from pyspectral_b200 import build
 

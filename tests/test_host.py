@@ -305,3 +305,79 @@ def test_tile_tuner_cache_roundtrip(tmp_path):
     assert load_tune_cache(p)[k]["tile"] == 2
     p.write_text("not json")
     assert load_tune_cache(p) == {}
+
+
+class _TunerLib:
+    """The calls a tuner makes, counted; one revision of the library."""
+
+    def __init__(self, revision):
+        self.revision, self.steps = revision, 0
+
+    def sp_source_revision(self):
+        return self.revision
+
+    def sp_batch_tile_supported(self, n, tile):
+        return 1
+
+    def sp_batch_step(self, h, stream):
+        self.steps += 1
+        return 0
+
+    sp_group_step = sp_batch_step
+
+    def sp_batch_prepare(self, h, stream):
+        return 0
+
+    def sp_batch_set_tile(self, h, tile):
+        return 0
+
+
+def _tuned(lib, path):
+    """(tile, work list) that a new tuner on the cache at ``path`` chooses with library ``lib``."""
+    from types import SimpleNamespace
+
+    from pyspectral_b200.ensemble import TileTuner
+
+    class Event:
+        def __init__(self, enable_timing):
+            pass
+
+        def record(self, stream):
+            self.at = lib.steps
+
+        def synchronize(self):
+            pass
+
+        def elapsed_time(self, other):
+            return 1.0
+
+    cuda = SimpleNamespace(get_device_name=lambda d: "GPU", current_stream=lambda d: None,
+                           Event=Event)
+    sc = SimpleNamespace(torch=SimpleNamespace(cuda=cuda), lib=lib, n=256, fp64=False, count=8,
+                         u0=SimpleNamespace(device=0), h=None, set_step=lambda *a: None,
+                         _check=lambda *a: None)
+    ens = SimpleNamespace(torch=sc.torch, lib=lib, device=0, classes=[sc], _group=None,
+                          _worklist_ok=lambda mt: True, _stream=lambda: None,
+                          _gcheck=lambda *a: None, set_worklist=lambda mt: None)
+    tuner = TileTuner(path)
+    return tuner.choose(sc, None), tuner.choose_worklist(ens)
+
+
+def test_tuned_choices_of_another_library_are_timed_again(tmp_path):
+    """A cached tile or work list holds for the kernels it was timed with: an entry without a
+    revision, or of another one, is timed again and replaced; the library's own is used."""
+    from pyspectral_b200.ensemble import load_tune_cache, save_tune_cache, tune_key
+
+    p = tmp_path / "tiles.json"
+    key, group = tune_key("GPU", 256, False, 8), "GPU|group|256fx8"
+    save_tune_cache(p, {key: {"tile": 4, "ms_per_step": {"4": 0.5}},
+                        group: {"worklist": 128, "ms_per_step": {"128": 0.5}}})
+    first = _TunerLib(b"r1")
+    assert _tuned(first, p) == (1, 0) and first.steps > 0  # equal times: the first candidate
+    assert load_tune_cache(p)[key]["revision"] == "r1"
+    assert load_tune_cache(p)[group]["revision"] == "r1"
+    again = _TunerLib(b"r1")
+    assert _tuned(again, p) == (1, 0) and again.steps == 0
+    later = _TunerLib(b"r2")
+    assert _tuned(later, p) == (1, 0) and later.steps == first.steps
+    assert load_tune_cache(p)[key]["revision"] == "r2"
