@@ -572,9 +572,10 @@ __device__ __forceinline__ void adam_update(int j, float g, int t, const AdamCfg
 // Sums the CTAs' partial rows: 32 parameters per CTA, warp g sums rows g, g + 8, .. of them (one
 // 128-byte access each) and the eight sums are added in order, so the gradient is
 // bit-reproducible.  (One thread per parameter over all the rows was a chain of 148 loads in 61
-// CTAs: 10.1 us, and the update 5.3 us after it; one launch of 8.4 us now, cold.)  The column kNParam is the step's loss.  ADAM: the same thread then updates
-// its parameter; `advance` moves the step counter on once every CTA has read it (the last CTA to
-// finish, by `ticket`).
+// CTAs: 10.1 us, and the update 5.3 us after it; one launch of 8.4 us now, cold.)  The column
+// kNParam is the step's loss.  ADAM: the same thread then updates
+// its parameter; `advance` moves the step counter on once every CTA has read it (the last one to
+// draw a `ticket`, in a warp that the update leaves idle).
 constexpr int kReduceRows = 8;
 template <bool ADAM>
 __global__ void __launch_bounds__(32 * kReduceRows)
@@ -605,9 +606,12 @@ __global__ void __launch_bounds__(32 * kReduceRows)
             loss_ring[step & (kLossRing - 1)] = s;
         }
     }
-    if (advance && threadIdx.x == 0) {
-        // this CTA's step was read before the barrier above
+    if (advance && threadIdx.x == 32) {
+        // this CTA's threads read the step before the barrier above; the fences order those
+        // reads, of every CTA, before the write
+        __threadfence();
         if (atomicAdd(ticket, 1u) == gridDim.x - 1) {
+            __threadfence();
             *step_dev = (int)step + 1;
             *ticket = 0;
         }
