@@ -195,19 +195,20 @@ __device__ __forceinline__ void dft8(E* x) {
     }
 }
 
+// n = 4 n1 + n2, k = k1 + 4 k2: inner DFT4 over n1 (column n2), twiddle w16^{n2 k1}, outer DFT4
+// over n2
 template <int DIR, typename E>
-__device__ __forceinline__ void dft16(E* x) {
-    // n = 4 n1 + n2, k = k1 + 4 k2: inner DFT4 over n1, twiddle w16^{n2 k1}, outer DFT4 over n2
-    E y[16];
-#pragma unroll
-    for (int n2 = 0; n2 < 4; ++n2) {
-        E a = x[n2], b = x[4 + n2], c = x[8 + n2], d = x[12 + n2];
-        dft4<DIR>(a, b, c, d);  // k1 = 0..3
-        y[n2 * 4 + 0] = a;
-        y[n2 * 4 + 1] = b;
-        y[n2 * 4 + 2] = c;
-        y[n2 * 4 + 3] = d;
-    }
+__device__ __forceinline__ void dft16_inner(const E* x, E* y, int n2) {
+    E a = x[n2], b = x[4 + n2], c = x[8 + n2], d = x[12 + n2];
+    dft4<DIR>(a, b, c, d);  // k1 = 0..3
+    y[n2 * 4 + 0] = a;
+    y[n2 * 4 + 1] = b;
+    y[n2 * 4 + 2] = c;
+    y[n2 * 4 + 3] = d;
+}
+
+template <int DIR, typename E>
+__device__ __forceinline__ void dft16_outer(E* x, E* y) {
     y[1 * 4 + 1] = rot16<DIR, 1>(y[1 * 4 + 1]);
     y[1 * 4 + 2] = rot16<DIR, 2>(y[1 * 4 + 2]);
     y[1 * 4 + 3] = rot16<DIR, 3>(y[1 * 4 + 3]);
@@ -228,6 +229,14 @@ __device__ __forceinline__ void dft16(E* x) {
     }
 }
 
+template <int DIR, typename E>
+__device__ __forceinline__ void dft16(E* x) {
+    E y[16];
+#pragma unroll
+    for (int n2 = 0; n2 < 4; ++n2) dft16_inner<DIR>(x, y, n2);
+    dft16_outer<DIR>(x, y);
+}
+
 // dft16<+1> of inputs with x[7] = 0 and x[15] = c r (a product of a real and a complex value),
 // x[15] holding the rounded product: where fx (fy) is set, the sums that take the product's real
 // (imaginary) part are fused multiply-adds of the unrounded product.
@@ -239,37 +248,13 @@ __device__ __forceinline__ void dft16_fused15(C* x, R c, C r, bool fx, bool fy) 
     const C a = eadd(x[3], x[11]), b = esub(x[3], x[11]);
     C y[16];
 #pragma unroll
-    for (int n2 = 0; n2 < 3; ++n2) {
-        C p = x[n2], q = x[4 + n2], u = x[8 + n2], w = x[12 + n2];
-        dft4<1>(p, q, u, w);
-        y[n2 * 4 + 0] = p;
-        y[n2 * 4 + 1] = q;
-        y[n2 * 4 + 2] = u;
-        y[n2 * 4 + 3] = w;
-    }
-    // a + x15, b - i x15, a - x15, b + i x15
+    for (int n2 = 0; n2 < 3; ++n2) dft16_inner<1>(x, y, n2);
+    // column 3: a + x15, b - i x15, a - x15, b + i x15
     y[12] = mk<R>(fma(mx, qx, a.x), fma(my, qy, a.y));
     y[13] = mk<R>(fma(my, qy, b.x), fma(-mx, qx, b.y));
     y[14] = mk<R>(fma(-mx, qx, a.x), fma(-my, qy, a.y));
     y[15] = mk<R>(fma(-my, qy, b.x), fma(mx, qx, b.y));
-    y[5] = rot16<1, 1>(y[5]);
-    y[6] = rot16<1, 2>(y[6]);
-    y[7] = rot16<1, 3>(y[7]);
-    y[9] = rot16<1, 2>(y[9]);
-    y[10] = rot16<1, 4>(y[10]);
-    y[11] = rot16<1, 6>(y[11]);
-    y[13] = rot16<1, 3>(y[13]);
-    y[14] = rot16<1, 6>(y[14]);
-    y[15] = rot16<1, 9>(y[15]);
-#pragma unroll
-    for (int k1 = 0; k1 < 4; ++k1) {
-        C p = y[k1], q = y[4 + k1], u = y[8 + k1], w = y[12 + k1];
-        dft4<1>(p, q, u, w);
-        x[k1 + 0] = p;
-        x[k1 + 4] = q;
-        x[k1 + 8] = u;
-        x[k1 + 12] = w;
-    }
+    dft16_outer<1>(x, y);
 }
 
 template <int R, int DIR, typename E>
