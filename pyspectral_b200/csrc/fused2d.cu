@@ -100,8 +100,8 @@ cudaError_t stream_attrs() {
     return cudaSuccess;
 }
 
-// Tile multipliers compiled for a grid: 1, 2, 4 up to n = 1024 (CTAs of at most 256 threads),
-// 1 above.
+// Tile multipliers compiled for a grid: 1, 2, 4 up to n = 1024 (CTAs of at most 256 threads in the
+// row pass and 512 in the column pass), 1 above.
 constexpr bool tile_ok(int n, int bx) { return bx == 1 || ((bx == 2 || bx == 4) && n <= 1024); }
 
 template <typename T, int N, int BX>

@@ -413,10 +413,12 @@ __device__ __forceinline__ void col_pass_cols(Pair<T>* __restrict__ X, int kc,
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 
-// Grids whose column pass gives each of a column's two sequences its own threads.  Above, the
-// streamed pass's prefetch buffer leaves no room for two exchange buffers, and it is faster than
-// this pass without the prefetch (2048^2 fp32 0.173 against 0.187 ms per step, 4096^2 0.651
-// against 0.833).  n = 16 keeps one thread per pair: its wavenumbers are constants of the unrolled
+// Grids whose column pass gives each of a column's two sequences its own threads.  Above, single
+// runs take the streamed pass, whose prefetch buffer leaves no room for two exchange buffers and
+// which is faster than this pass without the prefetch (2048^2 fp32 0.173 against 0.187 ms per step,
+// 4096^2 0.651 against 0.833).  Batches there take one thread per pair; against two threads, ms per
+// step: 4096^2 fp32, two members, 1.47 and 1.64, but 2048^2 fp32, four members, 0.710 and 0.664,
+// 2048^2 fp64, eight, 3.35 and 3.28, 4096^2 fp64, two, 3.71 and 3.20.  n = 16 keeps one thread per pair: its wavenumbers are constants of the unrolled
 // slots, and the sums there take other unrounded products than those stated below (20.8 us per
 // step, 16.7 with two threads, but other last bits).
 template <int N>
@@ -759,8 +761,12 @@ __global__ void __launch_bounds__(32) k_wait_probe(unsigned* __restrict__ err, u
 // Persistent passes of a batched group over a packed list of items, one launch per phase for
 // every size class: a CTA of MT threads takes items blockIdx.x, blockIdx.x + gridDim.x, ...;
 // an item is 16 MT / n rows (or columns) of one member, so every item fills the CTA and uses
-// the same shared memory whatever its n.  The row and column work per item is the single-run
-// passes' own (row_pass_rows, col_pass_cols).
+// the same shared memory whatever its n.  The work per item is row_pass_rows and col_pass_cols:
+// one thread per pair of a column, where launches per class have two (see split_columns), so that
+// lists are the slower form now.  Per group step, launches per class and list of 128 threads: one
+// member each of 128^2..1024^2 fp32 86 and 98 us, 4 each 217 and 241, 16 each 0.81 and 0.98 ms, 64
+// each 3.23 and 3.58; eight each of 32^2..128^2 (64 threads) 38 and 52 us; fp64, one each, 147 and
+// 282.
 template <int MT, int N>
 constexpr bool multi_fits() {
     return N >= 16 && (N & (N - 1)) == 0 && N / 16 <= MT && 16 * MT / N <= N;

@@ -150,9 +150,10 @@ constexpr int z_threads() { return sizeof(T) == 4 ? 128 : 64; }
 // XOR-swizzled by the row, so that eight lanes holding the same chunk of eight rows fall on
 // different banks; the transforms' exchanges reuse the tile's memory (n * 16 bytes per
 // sequence, the exchange of single complex values needs n * 8.5).
-// Bound now: HBM traffic in flight (512^3 fp32 Basdevant, one B200: inverse of 3 fields 0.768 ->
-// 0.388 ms = 4.6 TB/s, forward of 5 fields 0.943 -> 0.613 ms = 4.9 TB/s; 256^3 rotational 0.138
-// -> 0.074 and 0.070 -> 0.045 ms).
+// Bound now: the L1 data pipe (256^3 fp32: 71-78 % of its wavefronts inverse, 57-62 forward, most of
+// them shared) and HBM (52-64 and 57-67 %) at 18 warps per SM.  512^3 fp32 Basdevant, one B200:
+// inverse of 3 fields 0.768 -> 0.366 ms = 4.9 TB/s, forward of 5 fields 0.943 -> 0.569 ms = 5.3
+// TB/s; 256^3 rotational 0.147 -> 0.077 and 0.070 -> 0.039 ms.
 template <typename T, int N>
 struct YTile {
     using D = Dims<N>;
@@ -160,7 +161,8 @@ struct YTile {
     static constexpr int UN = 2 * QT;                            // transforms
     static constexpr int PT = UN * D::T;                         // threads
     // one warp per CTA at n <= 64, where CTAs of 128 threads leave SMs empty: fp32 Basdevant step
-    // 69.7 -> 65.6 us at 16^3, 71.7 -> 69.2 at 32^3 (the direct passes before the tiles: 69.7, 73.8)
+    // 69.7 -> 65.6 us at 16^3, 71.7 -> 69.2 at 32^3 (the direct passes before the tiles: 69.7 and
+    // 73.8)
     static constexpr int CTA = N <= 64 ? 32 : 128;
     static constexpr int KT = PT >= CTA ? 1 : CTA / PT;          // tiles per CTA
     static constexpr int THREADS = PT * KT;
@@ -502,14 +504,16 @@ __global__ void __launch_bounds__(z_threads<T>()) k3_z(Pair<T>* __restrict__ Bp,
 // row it will write (forward) or has read (inverse), so the rows are all the memory there is
 // and registers, not shared memory, set the resident CTAs.  The update's state and accumulator
 // are loaded one element ahead.  Bound: latency (load, transform, update, transform in a row) at
-// 18-20 warps per SM.  512^3 fp32 Basdevant 1.18 -> 1.11 ms, 256^3 rotational 0.140 -> 0.124
-// ms, 128^3 fp64 rotational 0.049 -> 0.038 ms per launch.
+// 18-20 warps per SM; in fp32 at 256^3 the L1 data pipe is 66-71 % busy, HBM 42-48 %.  512^3 fp32
+// Basdevant 1.18 -> 1.09 ms, 256^3 rotational 0.140 -> 0.120 ms, 128^3 fp64 rotational 0.049 ->
+// 0.038 ms per launch.
 template <typename T, int N, bool ROT>
 struct XPass {
     using D = Dims<N>;
     static constexpr int S = D::SEQ;
     // rotational form (six fields) at n = 512 in fp32: one kz pair per CTA and three CTAs per
-    // SM, which leaves the pass its registers (two pairs of 12 warps at two CTAs spill)
+    // SM (two pairs of 12 warps at two CTAs have 80 registers and spill much more: 1.57 against
+    // 1.29 ms when both were measured)
     static constexpr bool ONE_PAIR_ROT = ROT && sizeof(T) == 4 && S == 1;
     static constexpr int G = (S >= 2 || sizeof(T) == 8 || ONE_PAIR_ROT) ? 1 : 2;
     static constexpr int U = G * S;
@@ -518,12 +522,12 @@ struct XPass {
     static constexpr int ROW = D::KK;  // Pairs
     static constexpr size_t smem_bytes() { return (size_t)U * nslot<ROT>() * ROW * sizeof(Pair<T>); }
     static constexpr int UNITS = D::KK * D::NQ;
-    // fp64: two CTAs.  fp32: as many as 20 warps hold, 96 registers a thread, spilling up to 90
-    // bytes of it: at stage 1 against two CTAs without a spill, 128^3 Basdevant 19.0 and 21.2 us,
-    // 256^3 94 and 119, 256^3 rotational 119.3 and 120.2; three CTAs or the compiler's own
-    // registers (141-148, 96-114 at 512^3) 101 and more, 1.09 and 1.15-1.26 ms at 512^3 Basdevant.
-    // A grid that one CTA per SM holds (n <= 64) gains nothing from the warps: two CTAs there
-    // (64^3 Basdevant 9.9 -> 8.7 us, rotational 9.3 -> 8.8).
+    // fp64: two CTAs.  fp32: as many as 20 warps hold, 96 registers a thread, spilling up to 96
+    // bytes of them: at stage 1 against two CTAs without a spill, 128^3 Basdevant 19.0 and 21.2 us,
+    // 256^3 94 and 119, 256^3 rotational 119.3 and 120.2 (128^3 rotational 22.6 and 21.6, its step
+    // 231 with both).  With three CTAs or the compiler's own registers 256^3 Basdevant takes 101,
+    // 512^3 1.25 and 1.15 ms for 1.09.  A grid that one CTA per SM holds (n <= 64) gains nothing
+    // from the warps: two CTAs there (64^3 Basdevant 9.9 -> 8.7 us, rotational 9.3 -> 8.8).
     static constexpr int MIN_BLOCKS = sizeof(T) == 8 || (UNITS + U - 1) / U <= 148 ? 2 : 20 / WARPS;
     static_assert(FftPlan<N>::SMEM * sizeof(cplx<T>) <= ROW * sizeof(Pair<T>), "exchange fits a row");
 };
